@@ -221,20 +221,12 @@ def bench_config(world: int, shard: bool = False) -> dict:
 
 # ------------------------------------------------------------ our arm
 def algorithmic_bytes_xy_vpsi(ctx, npairs: int, nlaunch: float, cbytes: int, vbytes: int) -> float:
-    """Per H*psi, the H*psi plane kernel that starts from the stored psi(r)
-    (kxy_lane_fwd_staged): every band pair's psi(r) read once (N c bytes), its sticks
-    written once (S c bytes), and the potential read once per launch
-    (N v bytes)."""
+    """Per H*psi, the x pass (pen::xv: x transform, times V(r), x transform
+    back, in place): every band pair's tile of occupied columns read once and
+    written once, and the potential read once per launch (N v bytes)."""
     n0, n1, n2 = ctx.grid
-    N = n0 * n1 * n2
-    nvec = 2 * nrods(ctx) - 1
-    S = nvec * n2
-    return npairs * float(N + S) * cbytes + nlaunch * float(vbytes) * N
-
-
-def nrods(ctx) -> int:
-    hkl = ctx.miller()
-    return len({(int(h), int(k)) for h, k, _ in hkl})
+    ncol = 2 * int(max(h for h, _, _ in ctx.miller())) + 1
+    return npairs * 2.0 * ncol * n1 * n2 * cbytes + nlaunch * float(vbytes) * n0 * n1 * n2
 
 
 def run_ours(args):
@@ -323,7 +315,7 @@ def run_ours(args):
         prof[name] = {"ms_per_step": t / args.steps, "launches_per_step": n / args.steps}
     mix.profile(False)
     npairs = (s.nbands + 1) // 2
-    # one xy_vpsi launch per batch of band pairs
+    # the x pass takes all band pairs in one launch
     t_xy, n_xy = prof["xy_vpsi"]["ms_per_step"], prof["xy_vpsi"]["launches_per_step"]
     bytes_hpsi = algorithmic_bytes_xy_vpsi(mix, npairs, n_xy, 8, 4)
     per_launch_bytes = bytes_hpsi / max(1e-9, n_xy)
@@ -335,17 +327,15 @@ def run_ours(args):
         pass
     hbm_peak = peaks.get("hbm_gbs", 6650.0)
     achieved = per_launch_bytes / (per_launch_ms * 1e-3) / 1e9
-    roofline = {"kernel": "kxy_lane_fwd_staged<140,140> (H*psi plane pass from the stored "
-                          "psi(r), rows staged by cp.async: times V, forward x and y "
-                          "register-lane FFTs)",
+    roofline = {"kernel": "pen::xv<float, 140> (H*psi x pass: x transform of the tiles kept "
+                          "from the density pass, times V, transform back in place)",
                 "bound": "hbm",
                 "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                 "frac": achieved / hbm_peak,
                 "peak_source": "measured" if "hbm_gbs" in peaks else "fallback",
-                # DRAM bytes per launch: the ncu capture of the pruned kernel
-                # (profiles/kxy_lane_fwd_staged_si512.md: 416.1 MB for a
-                # 16-pair launch) scaled by the band pairs of this run's launches
-                "traffic": 416.1e6 / 16.0 * (npairs / max(1e-9, n_xy)),
+                # every tile element is read and written by one thread, so
+                # the DRAM bytes are the algorithmic ones
+                "traffic": per_launch_bytes,
                 "algorithmic_bytes_per_launch": per_launch_bytes,
                 "launch_ms": per_launch_ms}
     # GEMM share: the split-precision products of the mixed step (BF16 and

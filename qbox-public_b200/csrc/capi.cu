@@ -70,9 +70,9 @@ void free_cell(Context& c) {
   if (c.s_out) cudaStreamSynchronize(c.s_out);
   dfree(c.d_cin);
   dfree(c.d_cout);
-  if (c.d_psir) { cudaFree(c.d_psir); c.d_psir = nullptr; }
-  c.psir_bytes = 0;
-  c.psir_valid = false;
+  if (c.d_wtile) { cudaFree(c.d_wtile); c.d_wtile = nullptr; }
+  c.wtile_bytes = 0;
+  c.tile_valid = false;
   c.in_pending = c.finish_pending = false;
   free_mixed(c);
   free_mix(c);
@@ -164,15 +164,29 @@ void finish_step(Context& c, bool want_f, bool want_s) {
   if (want_s) finish_stress(c);
 }
 
+// However a step ends, no tile of its density pass is used by a later call.
+struct TileScope {
+  Context& c;
+  ~TileScope() {
+    c.tile_store = c.tile_use = c.tile_valid = false;
+    for (KPointSet& kp : c.kpts) kp.tile_valid = false;
+  }
+};
+
 // BOSampleStepper's electronic step (src/BOSampleStepper.cpp:795-1114 with
 // nite = 0), every operation on c.stream.
 void step_eager(Context& c, bool want_f, bool want_s, double* energies, double* fion) {
+  TileScope tiles{c};
   if (!c.kpts.empty()) {
     // k points off Gamma: the same sequence on the complex SlaterDets
     QBX_REQUIRE(!want_f && !want_s, 1, "forces and stress are not available at k points off Gamma");
+    c.tile_store = true;
     update_density_k(c);
+    c.tile_store = false;
     update_vhxc(c);
+    c.tile_use = true;
     energy_k(c, true);
+    c.tile_use = false;
     eigsum_k(c);
     readback(c, false);
     check_status(c);
@@ -184,15 +198,14 @@ void step_eager(Context& c, bool want_f, bool want_s, double* energies, double* 
     finish_theta(c);
     return;
   }
-  // psi(r) of the density pass is reused by the H*psi pass
-  c.psir_store = true;
+  // the tiles of the density pass are reused by the H*psi pass
+  c.tile_store = true;
   update_density(c);
-  c.psir_store = false;
+  c.tile_store = false;
   update_vhxc(c);
-  c.psir_use = true;
+  c.tile_use = true;
   energy(c, true, want_f);
-  c.psir_use = false;
-  c.psir_valid = false;
+  c.tile_use = false;
   if (want_s) compute_stress(c);
   launch_eigsum(c);
   readback(c, want_f);
@@ -220,8 +233,8 @@ long record_step(Context& c, bool want_f) {
   const long n0 = c.nlaunch;
   c.prof.on = false;
   c.capturing = true;
+  TileScope tiles{c};
   auto restore = [&]() {
-    c.psir_store = c.psir_use = c.psir_valid = false;
     c.capturing = false;
     c.prof.on = prof;
     c.extrapolate = extrap;
@@ -230,9 +243,13 @@ long record_step(Context& c, bool want_f) {
   try {
     if (!c.kpts.empty()) {
       // k points off Gamma: the same sequence on the complex SlaterDets
+      c.tile_store = true;
       update_density_k(c);
+      c.tile_store = false;
       update_vhxc(c);
+      c.tile_use = true;
       energy_k(c, true);
+      c.tile_use = false;
       eigsum_k(c);
       psda_update_k(c);
       enqueue_readback(c, false);
@@ -241,14 +258,13 @@ long record_step(Context& c, bool want_f) {
       c.nlaunch = n0;
       return k;
     }
-    c.psir_store = true;
+    c.tile_store = true;
     update_density(c);
-    c.psir_store = false;
+    c.tile_store = false;
     update_vhxc(c);
-    c.psir_use = true;
+    c.tile_use = true;
     energy(c, true, want_f);
-    c.psir_use = false;
-    c.psir_valid = false;
+    c.tile_use = false;
     psda_update(c, PSDA_PREC_FROM_ENERGY | PSDA_EIGSUM);
     enqueue_readback(c, want_f);
   } catch (...) {
@@ -525,8 +541,7 @@ int qbx_set_cell(qbx_context* h, const double cell[9], double ecut, int nst, con
     c.pair_batch = (int)std::max<size_t>(1, std::min<size_t>(npairs, ((size_t)4 << 30) / per_pair));
     QBX_CUDA(cudaMalloc(&c.d_zbuf, per_pair * c.pair_batch));
     c.zbuf_bytes = per_pair * c.pair_batch;
-    // the specialised FFTs work through a smaller stick buffer that can stay
-    // in L2 between the z and plane kernels (64 MB unless overridden)
+    // stick buffer of the line passes, in batches of band pairs
     {
       size_t mb = 256;
       if (const char* e = std::getenv("QBX_FAST_ZBUF_MB")) mb = std::max(1, std::atoi(e));
@@ -536,24 +551,7 @@ int qbx_set_cell(qbx_context* h, const double cell[9], double ecut, int nst, con
       c.d_vr32 = dalloc<float>(N);
       c.fast_fft = true;
       if (const char* e = std::getenv("QBX_FAST_FFT")) c.fast_fft = std::atoi(e) != 0;
-      if (const char* e = std::getenv("QBX_FAST_WARPS")) c.fast_warps = std::max(1, std::min(16, std::atoi(e)));
-      if (const char* e = std::getenv("QBX_FAST_RODS")) c.fast_rods = std::max(1, std::min(32, std::atoi(e)));
-      if (const char* e = std::getenv("QBX_FAST_CHUNKS")) c.fast_chunks = std::max(1, std::atoi(e));
-      c.fast_batch = 16;
-      if (const char* e = std::getenv("QBX_FAST_BATCH")) c.fast_batch = std::max(0, std::atoi(e));
-      if (const char* e = std::getenv("QBX_FAST_LANE_SHAPE"))
-        c.fast_lane_shape = std::max(-1, std::min(6, std::atoi(e)));
-      if (const char* e = std::getenv("QBX_FAST_DENSITY_LANE_SHAPE"))
-        c.fast_density_lane_shape = (std::atoi(e) == 3 || std::atoi(e) >= 5) && std::atoi(e) <= 8
-                                        ? std::atoi(e) : 2;
-      if (const char* e = std::getenv("QBX_PSIR")) c.psir_mode = std::atoi(e) != 0 ? 1 : 0;
-      if (const char* e = std::getenv("QBX_FWD_STAGED")) c.fast_fwd_staged = std::atoi(e) != 0 ? 1 : 0;
-      if (const char* e = std::getenv("QBX_FFT_PRUNE")) c.fast_prune = std::atoi(e) != 0 ? 1 : 0;
-      if (const char* e = std::getenv("QBX_ZLANE")) c.fast_zlane = std::max(0, std::min(3, std::atoi(e)));
-      if (const char* e = std::getenv("QBX_FWD_PAIRS_PER_CTA"))
-        c.fast_fwd_ppc = std::max(1, std::min(64, std::atoi(e)));
-      if (const char* e = std::getenv("QBX_FAST_VPSI_SHAPE"))
-        c.fast_vpsi_shape = std::max(0, std::min(2, std::atoi(e)));
+      if (const char* e = std::getenv("QBX_PSIR")) c.wtile_mode = std::atoi(e) != 0 ? 1 : 0;
     }
     c.species.clear();
     c.tau.clear();
@@ -1286,19 +1284,11 @@ int qbx_autotune(qbx_context* h, char* report, int report_len) {
     check_ready(c, true);
     std::vector<std::pair<std::string, double>> log;
     drop_graphs(c);   // the launch shapes may change
-    autotune_fft(c, &log);
+    const std::string pick = autotune_fft(c, &log);
     if (report && report_len > 0) {
       std::string r;
       for (auto& e : log) r += e.first + ": " + std::to_string(e.second) + " ms\n";
-      r += "chosen: lane " + std::to_string(c.fast_lane_shape) + ", warp " +
-           std::to_string(c.fast_vpsi_shape) + ", density lane " +
-           std::to_string(c.fast_density_lane_shape) + " x " + std::to_string(c.fast_chunks) +
-           ", pairs " +
-           std::to_string(c.fast_batch) + ", rods " + std::to_string(c.fast_rods) +
-           ", z lanes " + std::to_string(c.fast_zlane) + ", pruned xy " +
-           std::to_string(c.fast_prune && c.dws.xw <= prune_width(c.dws.n0) &&
-                          c.dws.yw <= prune_width(c.dws.n1)) +
-           " z " + std::to_string(c.fast_prune && c.dws.zw <= prune_width(c.dws.n2)) + "\n";
+      r += "chosen: " + pick + "\n";
       std::strncpy(report, r.c_str(), (size_t)report_len - 1);
       report[report_len - 1] = 0;
     }

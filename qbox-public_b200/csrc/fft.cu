@@ -27,10 +27,11 @@
 // All 1-D FFTs are mixed-radix (2,3,4,5,7,11) self-sorting Stockham passes
 // over shared memory with a twiddle table exp(+2 pi i k/n) built in FP64.
 #include <algorithm>
+#include <complex>
 #include <cstdio>
 #include <vector>
 
-#include "fft_fast.cuh"
+#include "fft_pencil.cuh"
 #include "qbx_internal.h"
 
 namespace qbx {
@@ -511,6 +512,11 @@ void upload_sticks(DeviceSticks& d, const Basis& b) {
   d.stick_y = dupload(b.stick_y);
   d.stick_col = dupload(b.stick_col);
   d.col_x = dupload(b.col_x);
+  {
+    std::vector<int> xc(b.n0, -1);
+    for (int i = 0; i < b.ncol; i++) xc[b.col_x[i]] = i;
+    d.xcol = dupload(xc);
+  }
   d.ip = dupload(b.ip);
   d.im = dupload(b.im);
   {
@@ -527,6 +533,13 @@ void upload_sticks(DeviceSticks& d, const Basis& b) {
   d.px = make_plan(b.n0);
   d.py = make_plan(b.n1);
   d.pz = make_plan(b.n2);
+  d.gain32 = 1.0;
+  double gain = 1.0;
+  for (int i = 0; i < 3; i++) {
+    const int n3[3] = {b.n0, b.n1, b.n2};
+    if (i == 0 || n3[i] != n3[i - 1]) gain = pencil_length(n3[i]) ? pencil_gain_fp32(n3[i]) : 1.0;
+    d.gain32 *= gain;
+  }
   const int n[3] = {b.n0, b.n1, b.n2};
   for (int a = 0; a < 3; a++) {
     std::vector<double2> t = twiddle_table(n[a]);
@@ -538,7 +551,7 @@ void upload_sticks(DeviceSticks& d, const Basis& b) {
 void free_sticks(DeviceSticks& d) {
   for (int a = 0; a < 3; a++) dfree(d.tw[a]);
   dfree(d.rod_first); dfree(d.rod_lmin); dfree(d.rod_size);
-  dfree(d.stick_y); dfree(d.stick_col); dfree(d.col_x);
+  dfree(d.stick_y); dfree(d.stick_col); dfree(d.col_x); dfree(d.xcol);
   dfree(d.ip); dfree(d.im);
   dfree(d.colmap);
 }
@@ -712,6 +725,228 @@ k_zfft_fwd_k(const double2* __restrict__ zbuf, int ngw, int band0, DeviceSticks 
   }
 }
 
+// ------------------------------------------------------- line-pass FFTs
+// (fft_pencil.cuh) The grids of the plane-free passes: z fastest.
+// x-fastest grid <-> [x][y][z], 32 x 32 tiles of (x, z) at each y
+template <typename A, typename B, bool ADD>
+__global__ void __launch_bounds__(256)
+k_grid_to_zfast(const A* __restrict__ in, int n0, int n1, int n2, bool to_zfast,
+                B* __restrict__ out) {
+  __shared__ B t[32][33];
+  const int x0 = blockIdx.x * 32, z0 = blockIdx.y * 32, y = blockIdx.z;
+  const int a = threadIdx.x & 31, b = threadIdx.x >> 5;
+  for (int i = b; i < 32; i += 8) {
+    const int x = to_zfast ? x0 + a : x0 + i, z = to_zfast ? z0 + i : z0 + a;
+    if (x < n0 && z < n2)
+      t[i][a] = (B)in[to_zfast ? ((size_t)z * n1 + y) * n0 + x : ((size_t)x * n1 + y) * n2 + z];
+  }
+  __syncthreads();
+  for (int i = b; i < 32; i += 8) {
+    const int x = to_zfast ? x0 + i : x0 + a, z = to_zfast ? z0 + a : z0 + i;
+    if (x < n0 && z < n2) {
+      B* o = out + (to_zfast ? ((size_t)x * n1 + y) * n2 + z : ((size_t)z * n1 + y) * n0 + x);
+      *o = ADD ? *o + t[a][i] : t[a][i];
+    }
+  }
+}
+
+template <typename T>
+static bool pencil_run(Context& ctx, int n, const pen::Args& a) {
+  return pencil_0<T>(ctx, n, a) || pencil_1<T>(ctx, n, a) || pencil_2<T>(ctx, n, a) ||
+         pencil_3<T>(ctx, n, a) || pencil_4<T>(ctx, n, a) || pencil_5<T>(ctx, n, a) ||
+         pencil_6<T>(ctx, n, a) || pencil_7<T>(ctx, n, a);
+}
+
+// matrix of the FP32 register DFT of m points (row-major, the roots as the
+// kernels round them)
+using zmat = std::vector<std::complex<double>>;
+static zmat roots_fp32(int n) {
+  zmat r(n);
+  for (int k = 0; k < n; k++)
+    r[k] = {(double)(float)lane::cx_cos(k, n), (double)(float)lane::cx_sin(k, n)};
+  return r;
+}
+static zmat dft_fp32(int m) {
+  zmat f((size_t)m * m);
+  const zmat w = roots_fp32(m);
+  const int r1 = lane::first_radix(m);
+  if (m == r1) {
+    for (int k = 0; k < m; k++)
+      for (int j = 0; j < m; j++) f[(size_t)k * m + j] = w[(j * k) % m];
+    return f;
+  }
+  const int q1 = m / r1;
+  const zmat a = dft_fp32(q1), b = dft_fp32(r1);
+  for (int s = 0; s < r1; s++)
+    for (int q = 0; q < q1; q++)
+      for (int r = 0; r < r1; r++)
+        for (int k = 0; k < q1; k++)
+          f[(size_t)(q + q1 * s) * m + r + r1 * k] =
+              b[(size_t)s * r1 + r] * w[r * q] * a[(size_t)q * q1 + k];
+  return f;
+}
+
+double pencil_gain_fp32(int n) {
+  const int r1 = pen::fac(n).r1, r2 = pen::fac(n).r2, pw = prune_width(n);
+  const zmat a = dft_fp32(r1), b = dft_fp32(r2), w = roots_fp32(n);
+  zmat bn(r2, 0.0);                        // column norms of the second DFT
+  for (int j = 0; j < r2; j++)
+    for (int m = 0; m < r2; m++) bn[j] += std::norm(b[(size_t)m * r2 + j]);
+  double sum = 0.0;
+  int count = 0;
+  for (int x = 0; x < n; x++) {
+    if (x > pw && x < n - pw) continue;
+    const int j = x % r2, q = x / r2;
+    for (int k = 0; k < r1; k++)
+      sum += bn[j].real() * std::norm(w[j * k]) * std::norm(a[(size_t)k * r1 + q]);
+    count++;
+  }
+  return sum / ((double)count * n);
+}
+
+// bytes of one slot's sticks and of its tile
+static size_t pencil_stick_bytes(const DeviceSticks& g, bool fp32) {
+  return (fp32 ? sizeof(float2) : sizeof(double2)) * (size_t)g.n2 * g.nvec;
+}
+static size_t pencil_tile_bytes(const DeviceSticks& g, bool fp32) {
+  return (fp32 ? sizeof(float2) : sizeof(double2)) * (size_t)g.n2 * g.ncol * g.n1;
+}
+
+// The line passes take every grid whose lengths are compiled, whose sphere
+// lies within prune_width on each axis and whose slot fits the stick buffer;
+// the rest runs the runtime-radix kernels above.
+static bool pencil_ok(const Context& ctx, const DeviceSticks& g, bool fp32) {
+  return ctx.fast_fft && ctx.d_zfast && pencil_length(g.n0) && pencil_length(g.n1) &&
+         pencil_length(g.n2) && g.xw <= prune_width(g.n0) && g.yw <= prune_width(g.n1) &&
+         g.zw <= prune_width(g.n2) &&
+         pencil_stick_bytes(g, fp32) + pencil_tile_bytes(g, fp32) <= ctx.zfast_bytes;
+}
+
+// The buffer that keeps every slot's tile (`need` bytes): allocated, outside
+// stream capture, when `keep` asks for it and the device has room; without
+// `keep` only a buffer that is there already.  Null: no such buffer, and the
+// tiles go through the stick buffer in batches.
+static void* tile_area(Context& ctx, size_t need, bool keep) {
+  if (ctx.d_wtile && ctx.wtile_bytes >= need) return ctx.d_wtile;
+  if (!keep || ctx.wtile_mode == 0 || ctx.capturing) return nullptr;
+  size_t freeb = 0, total = 0;
+  QBX_CUDA(cudaMemGetInfo(&freeb, &total));
+  if (freeb < need + ((size_t)4 << 30)) {
+    if (ctx.wtile_mode < 0) ctx.wtile_mode = 0;   // no room: transform twice from now on
+    return nullptr;
+  }
+  if (ctx.d_wtile) cudaFree(ctx.d_wtile);
+  ctx.d_wtile = nullptr;
+  QBX_CUDA(cudaMalloc(&ctx.d_wtile, need));
+  ctx.wtile_bytes = need;
+  return ctx.d_wtile;
+}
+
+// Slots first ... first + nslots of one wavefunction block (band pairs, or
+// bands of a k point with `complex_basis`) through the line passes.  Density:
+// added into rho (x fastest; `add`) or stored there.  H psi: hc = 1/2 g2 c + V
+// psi.  area: room for the tiles of all these slots (then the x pass is one
+// launch, and with `have` the tiles are those of the density pass), or null:
+// sticks and tiles in batches through the stick buffer.
+template <typename T>
+static void pencil_pass(Context& ctx, const DeviceSticks& g, bool complex_basis, int op,
+                        const double* c, int ngw, const double* g2, const double* v, double* rho,
+                        bool add, const double* w, int nw, double* hc, void* area, bool have,
+                        int first, int nslots) {
+  using C = typename Cplx<T>::t;
+  const size_t N = ctx.N();
+  const dim3 tg((g.n0 + 31) / 32, (g.n2 + 31) / 32, g.n1);
+  pen::Args a;
+  a.g = g;
+  for (int i = 0; i < 3; i++) a.tw[i] = g.tw[i];
+  a.c = (const double2*)c;
+  a.hc = (double2*)hc;
+  a.g2 = g2;
+  // FP32: the gain of the rounded roots taken out (as 1 in FP64), the weights
+  // in units of 1/Omega so that whole occupations are exact
+  const double gain = sizeof(T) == 4 ? g.gain32 : 1.0;
+  a.scale = 1.0 / ((double)N * gain);
+  a.wunit = sizeof(T) == 4 ? 1.0 / ctx.wb.omega : 1.0;
+  a.wout = a.wunit / gain;
+  a.ngw = ngw;
+  a.nst = ctx.nst;
+  a.w = w;
+  a.nw = nw;
+  a.rho = (double*)ctx.d_grid;              // density and V(r), z fastest
+  T* vt = (T*)((double*)ctx.d_grid + N);
+  a.v = vt;
+  a.stream = ctx.stream;
+  if (op == OP_VPSI) {
+    k_grid_to_zfast<double, T, false><<<tg, 256, 0, ctx.stream>>>(v, g.n0, g.n1, g.n2, true, vt);
+    QBX_LAUNCHED(ctx);
+  }
+  const size_t sb = pencil_stick_bytes(g, sizeof(T) == 4), tb = pencil_tile_bytes(g, sizeof(T) == 4);
+  const int batch = (int)std::min<size_t>(nslots, ctx.zfast_bytes / (area ? sb : sb + tb));
+  const int xcta = (g.n1 * g.n2 + 15) / 16, ycta = (g.ncol * g.n2 + 15) / 16;
+  auto pass = [&](int n, int what, int chunks, const char* name) {
+    ProfScope ps(ctx, name);
+    a.op = what;
+    a.chunks = chunks;
+    QBX_REQUIRE(pencil_run<T>(ctx, n, a), 21, "no line kernel of this length");
+  };
+  auto slots = [&](int s0, int ns) {
+    a.first = first + s0;
+    a.nslots = ns;
+    a.sticks = ctx.d_zfast;
+    a.tile = area ? (void*)((C*)area + s0 * (tb / sizeof(C)))
+                  : (void*)((C*)ctx.d_zfast + batch * (sb / sizeof(C)));
+  };
+  // CTAs per set of lines: enough for several per SM.  A CTA of the y passes
+  // takes up to 4 slots, one of the x passes up to 16 (the density sums that
+  // many slots in the context's precision before the FP64 sum)
+  auto chunks = [&](int ns, int cta, int most) {
+    return std::min(ns, std::max((ns + most - 1) / most, (1184 + cta - 1) / cta));
+  };
+  auto back = [&](int s0, int ns) {
+    slots(s0, ns);
+    pass(g.n2, complex_basis ? pen::ZBK : pen::ZB, 1, "zfft_bwd");
+    pass(g.n1, pen::YB, chunks(ns, ycta, 4), "y_bwd");
+  };
+  auto forth = [&](int s0, int ns) {
+    slots(s0, ns);
+    pass(g.n1, pen::YF, chunks(ns, ycta, 4), "y_fwd");
+    pass(g.n2, complex_basis ? pen::ZFK : pen::ZF, 1, "zfft_fwd");
+  };
+  auto x = [&](int s0, int ns) {
+    slots(s0, ns);
+    const int ch = chunks(ns, xcta, 16);
+    if (op == OP_DENSITY) {
+      a.rho_set = s0 == 0 && ch == 1;
+      if (s0 == 0 && !a.rho_set)
+        QBX_CUDA(cudaMemsetAsync(a.rho, 0, N * sizeof(double), ctx.stream));
+      pass(g.n0, pen::XD, ch, "xy_density");
+    } else {
+      pass(g.n0, pen::XV, ch, "xy_vpsi");
+    }
+  };
+  for (int s0 = 0; s0 < nslots; s0 += batch) {
+    const int ns = std::min(batch, nslots - s0);
+    if (!have) back(s0, ns);
+    if (area) continue;
+    x(s0, ns);
+    if (op == OP_VPSI) forth(s0, ns);
+  }
+  if (area) {
+    x(0, nslots);
+    for (int s0 = 0; op == OP_VPSI && s0 < nslots; s0 += batch)
+      forth(s0, std::min(batch, nslots - s0));
+  }
+  if (op == OP_DENSITY) {
+    if (add)
+      k_grid_to_zfast<double, double, true><<<tg, 256, 0, ctx.stream>>>(a.rho, g.n0, g.n1, g.n2,
+                                                                        false, rho);
+    else
+      k_grid_to_zfast<double, double, false><<<tg, 256, 0, ctx.stream>>>(a.rho, g.n0, g.n1, g.n2,
+                                                                         false, rho);
+    QBX_LAUNCHED(ctx);
+  }
+}
+
 static constexpr int kRodsPerCtaK = 2 * kRodsPerCta;   // one line per rod
 
 // bands of a k point per pass through the context's stick buffer
@@ -724,6 +959,23 @@ static int kbands_per_batch(const Context& ctx, const KPointSet& kp) {
 
 static void staged_k(Context& ctx, KPointSet& kp, int op, const double* v, double* rho) {
   const DeviceSticks& g = kp.dks;
+  if (pencil_ok(ctx, g, false)) {
+    // tiles of all k points one after the other
+    size_t off = 0, need = 0;
+    bool all = true;
+    for (KPointSet& q : ctx.kpts) {
+      if (&q == &kp) off = need;
+      need += pencil_tile_bytes(q.dks, false) * ctx.nst;
+      all = all && pencil_ok(ctx, q.dks, false);
+    }
+    char* area = all ? (char*)tile_area(ctx, need, op == OP_DENSITY && ctx.tile_store) : nullptr;
+    const bool have = op == OP_VPSI && area && ctx.tile_use && kp.tile_valid;
+    // the weights are two per band, both the band's
+    pencil_pass<double>(ctx, g, true, op, kp.d_c, kp.kb.ng, kp.d_g2, v, rho, true, kp.d_w2,
+                        2 * ctx.nst, kp.d_hc, area ? area + off : nullptr, have, 0, ctx.nst);
+    kp.tile_valid = op == OP_DENSITY && area && ctx.tile_store;
+    return;
+  }
   cudaStream_t st = ctx.stream;
   double2* zbuf = (double2*)ctx.d_zbuf;
   const int ngw = kp.kb.ng;
@@ -784,102 +1036,43 @@ void launch_vpsi_k(Context& ctx, KPointSet& kp, const double* v) {
 
 static int nblk(size_t n);
 
-__global__ void k_to_float(const double* __restrict__ x, size_t n, float* __restrict__ y) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x)
-    y[i] = (float)x[i];
-}
-
-// The specialised kernels of fft_fast_*.cu in batches of band pairs through
-// ctx.d_zfast; false when the grid has none.
-// the psi(r) buffer (FP32, every band pair on the whole grid), allocated
-// outside stream capture when the device has room for it
-static bool psir_ready(Context& ctx) {
-  if (ctx.psir_mode == 0 || ctx.precision != MIXED || ctx.fast_lane_shape < 0) return false;
-  const size_t need = (size_t)((ctx.nst + 1) / 2) * ctx.N() * sizeof(float2);
-  if (ctx.d_psir && ctx.psir_bytes >= need) return true;
-  if (ctx.capturing) return false;
-  size_t freeb = 0, total = 0;
-  QBX_CUDA(cudaMemGetInfo(&freeb, &total));
-  if (freeb < need + ((size_t)4 << 30)) {
-    if (ctx.psir_mode < 0) ctx.psir_mode = 0;   // no room: recompute psi(r) from now on
-    return false;
-  }
-  if (ctx.d_psir) cudaFree(ctx.d_psir);
-  QBX_CUDA(cudaMalloc(&ctx.d_psir, need));
-  ctx.psir_bytes = need;
-  return true;
-}
-
-static bool staged_fast(Context& ctx, int op, const double* c, const double* v, double* rho,
-                        const double* w, double* hc) {
-  if (!ctx.fast_fft || !ctx.d_zfast) return false;
+// This GPU's band pairs of c through the line passes; false when the grid is
+// not theirs.  The tiles of a density pass are kept for the H psi pass of the
+// same step where the step functions ask for it (tile_store, tile_use).
+static bool staged_pencil(Context& ctx, int op, const double* c, const double* v, double* rho,
+                          const double* w, double* hc) {
+  const bool fp32 = ctx.precision == MIXED;
   const DeviceSticks& g = ctx.dws;
-  fast::StagedArgs a{};
-  a.op = (op == OP_DENSITY) ? fast::XY_DENSITY : fast::XY_VPSI;
-  a.c = c;
-  a.rho = rho;
-  a.w = w;
-  a.hc = hc;
-  a.nst = ctx.nst;
-  a.zbuf = ctx.d_zfast;
-  a.twx = twiddles(ctx, 0);
-  a.twy = twiddles(ctx, 1);
-  a.twz = twiddles(ctx, 2);
-  a.rods_per_cta = ctx.fast_rods;
-  a.xy_warps = ctx.fast_warps;
-  a.vpsi_shape = ctx.fast_vpsi_shape;
-  a.lane_shape = ctx.fast_lane_shape;
-  a.density_lane_shape = ctx.fast_density_lane_shape;
-  a.density_chunks = ctx.fast_chunks;
-  a.fwd_pairs_per_cta = ctx.fast_fwd_ppc;
-  a.zlane = ctx.fast_zlane;
-  a.fwd_staged = ctx.fast_fwd_staged;
-  a.prune = ctx.fast_prune;
-  a.v = v;
-  a.psir = nullptr;
-  if (op == OP_DENSITY) {
-    ctx.psir_valid = false;
-    if (ctx.psir_store && psir_ready(ctx)) a.psir = ctx.d_psir;
-  } else if (ctx.psir_use && ctx.psir_valid && ctx.psir_src == c) {
-    a.psir = ctx.d_psir;
-  }
-  if (op == OP_VPSI && ctx.precision == MIXED) {
-    const size_t N = ctx.N();
-    k_to_float<<<nblk(N), 256, 0, ctx.stream>>>(v, N, ctx.d_vr32);
-    QBX_LAUNCHED(ctx);
-    a.v = ctx.d_vr32;
-  }
-  const size_t limit = (size_t)max_smem_optin(ctx.device);
+  if (!pencil_ok(ctx, g, fp32)) return false;
   int plo = 0, phi = 0;
-  shard_pairs(ctx, plo, phi);            // this GPU's band pairs
-  const int npairs = phi - plo;
-  const size_t per_pair = (ctx.precision == MIXED ? sizeof(float2) : sizeof(double2)) *
-                          (size_t)g.n2 * g.nvec;
-  int batch = (int)std::min<size_t>(std::max(npairs, 1), ctx.zfast_bytes / per_pair);
-  if (ctx.fast_batch > 0) batch = std::min(batch, ctx.fast_batch);
-  QBX_REQUIRE(batch >= 1, 21, "stick buffer of the specialised FFTs holds no band pair");
-  bool first = true;
-  for (int p0 = plo; p0 < phi; p0 += batch) {
-    a.pair0 = p0;
-    a.npairs = std::min(batch, phi - p0);
-    const bool ok = fast_staged_a(ctx, a, limit) || fast_staged_b(ctx, a, limit);
-    if (!ok) {
-      QBX_REQUIRE(first, 21, "specialised FFT kernels unavailable after the first batch");
-      return false;
-    }
-    first = false;
+  shard_pairs(ctx, plo, phi);
+  const bool keep = op == OP_DENSITY && ctx.tile_store;
+  const bool have = op == OP_VPSI && ctx.tile_use && ctx.tile_valid && ctx.tile_src == c;
+  ctx.tile_valid = false;
+  if (phi <= plo) {
+    if (op == OP_DENSITY)
+      QBX_CUDA(cudaMemsetAsync(rho, 0, ctx.N() * sizeof(double), ctx.stream));
+    return true;
   }
-  if (op == OP_DENSITY && a.psir) {
-    ctx.psir_valid = true;
-    ctx.psir_src = c;
+  void* area = tile_area(ctx, pencil_tile_bytes(g, fp32) * (phi - plo), keep);
+  auto run = [&](auto t) {
+    pencil_pass<decltype(t)>(ctx, g, false, op, c, ctx.wb.ng, ctx.d_g2_w, v, rho, false, w,
+                             ctx.nst, hc, area, have, plo, phi - plo);
+  };
+  if (fp32) run(0.f);
+  else run(0.0);
+  if (keep && area) {
+    ctx.tile_valid = true;
+    ctx.tile_src = c;
   }
   return true;
 }
 
 static void staged(Context& ctx, int op, const double* c, const double* v, double* rho,
                    const double* w, double* hc) {
-  if (staged_fast(ctx, op, c, v, rho, w, hc)) return;
+  if (staged_pencil(ctx, op, c, v, rho, w, hc)) return;
+  if (op == OP_DENSITY)
+    QBX_CUDA(cudaMemsetAsync(rho, 0, ctx.N() * sizeof(double), ctx.stream));
   int plo = 0, phi = 0;
   shard_pairs(ctx, plo, phi);
   for (int p0 = plo; p0 < phi; p0 += ctx.pair_batch) {
@@ -895,7 +1088,6 @@ static void staged(Context& ctx, int op, const double* c, const double* v, doubl
 // transforms its own pairs; the density is then summed over the GPUs and
 // the H*psi blocks gathered, so every GPU continues with the whole of both.
 void launch_density(Context& ctx, const double* c, double* rho) {
-  QBX_CUDA(cudaMemsetAsync(rho, 0, ctx.N() * sizeof(double), ctx.stream));
   staged(ctx, OP_DENSITY, c, nullptr, rho, density_weights(ctx), nullptr);
   if (ctx.shard_comm) shard_sum(ctx, rho, ctx.N());
 }
@@ -905,6 +1097,18 @@ void launch_vpsi(Context& ctx, const double* c, const double* v, double* hc) {
   if (ctx.shard_comm) shard_gather_bands(ctx, hc);
 }
 
+static bool pencil_grid(Context& ctx, int n, double2* grid, const double2* tw, int inner,
+                        int nlines, int dir) {
+  return pencil_grid_0(ctx, n, grid, tw, inner, nlines, dir) ||
+         pencil_grid_1(ctx, n, grid, tw, inner, nlines, dir) ||
+         pencil_grid_2(ctx, n, grid, tw, inner, nlines, dir) ||
+         pencil_grid_3(ctx, n, grid, tw, inner, nlines, dir) ||
+         pencil_grid_4(ctx, n, grid, tw, inner, nlines, dir) ||
+         pencil_grid_5(ctx, n, grid, tw, inner, nlines, dir) ||
+         pencil_grid_6(ctx, n, grid, tw, inner, nlines, dir) ||
+         pencil_grid_7(ctx, n, grid, tw, inner, nlines, dir);
+}
+
 // full-grid transform of `grid` on the geometry of d (sizes, twiddles)
 static void grid_fft_on(Context& ctx, const DeviceSticks& b, double2* grid, int dir) {
   ProfScope ps(ctx, "grid_fft");
@@ -912,11 +1116,10 @@ static void grid_fft_on(Context& ctx, const DeviceSticks& b, double2* grid, int 
   const int L = 16;
   for (int axis = 0; axis < 3; axis++) {
     const double2* tw = b.tw[axis];
-    // compile-time lengths: warp FFTs on coalesced tiles (fft_fast.cuh)
-    if (ctx.fast_fft &&
-        (fast_grid_lines_a(ctx, grid, b.n0, b.n1, b.n2, axis, dir, tw) ||
-         fast_grid_lines_b(ctx, grid, b.n0, b.n1, b.n2, axis, dir, tw)))
-      continue;
+    // compiled lengths: register lines (fft_pencil.cuh)
+    const int inner = axis == 0 ? 1 : axis == 1 ? b.n0 : b.n0 * b.n1;
+    const int nlines = axis == 0 ? b.n1 * b.n2 : axis == 1 ? b.n0 * b.n2 : b.n0 * b.n1;
+    if (ctx.fast_fft && pencil_grid(ctx, n[axis], grid, tw, inner, nlines, dir)) continue;
     const RadixPlan p = make_plan(n[axis]);
     int nblocks;
     if (axis == 0) nblocks = (b.n1 * b.n2 + L - 1) / L;
@@ -1153,121 +1356,49 @@ void density_with_buffers(Context& ctx, const double* c, int nst, const double* 
 namespace qbx {
 
 // ------------------------------------------------------------ autotuner
-// Picks the staged-FFT launch configuration (plane-kernel family and CTA
-// shape for H*psi and for the density, band pairs per launch, rods per z
-// CTA) for this context's grid, basis and precision by timing the
-// candidates on the context's own wavefunctions and potential, one
-// parameter at a time in that order.  Results go to ctx.fast_*; the chosen
-// values and timings are appended to `log`.
-void autotune_fft(Context& ctx, std::vector<std::pair<std::string, double>>* log) {
+// Picks the staged-FFT kernels for this context's grid, basis and precision
+// by timing the candidates on the context's own wavefunctions and potential:
+// the line passes (fft_pencil.cuh), where they take the grid, or the
+// runtime-radix kernels.  Returns the choice's name; the timings are
+// appended to `log`.
+std::string autotune_fft(Context& ctx, std::vector<std::pair<std::string, double>>* log) {
   QBX_REQUIRE(ctx.have_cell && ctx.d_zfast, 7, "autotune needs a cell");
-  const size_t N = ctx.N();
-  double* rho_tmp = dalloc<double>(N);
-  double* hc_tmp = ctx.d_ctmp;
-  cudaEvent_t e0, e1;
-  QBX_CUDA(cudaEventCreate(&e0));
-  QBX_CUDA(cudaEventCreate(&e1));
-  auto time_ms = [&](auto fn) {
-    fn();   // warm-up (function attributes, caches)
-    QBX_CUDA(cudaEventRecord(e0, ctx.stream));
-    fn();
-    QBX_CUDA(cudaEventRecord(e1, ctx.stream));
-    QBX_CUDA(cudaEventSynchronize(e1));
-    float ms = 0.f;
-    QBX_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-    return (double)ms;
+  double* rho_tmp = dalloc<double>(ctx.N());
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  auto release = [&]() {
+    if (e0) cudaEventDestroy(e0);
+    if (e1) cudaEventDestroy(e1);
+    dfree(rho_tmp);
   };
-  auto vpsi = [&]() { launch_vpsi(ctx, ctx.d_c, ctx.d_vr, hc_tmp); };
-  auto dens = [&]() { launch_density(ctx, ctx.d_c, rho_tmp); };
-  auto note = [&](const std::string& what, double ms) {
-    if (log) log->push_back({what, ms});
-  };
+  const bool line = pencil_ok(ctx, ctx.dws, ctx.precision == MIXED);
+  double best = 1e30;
+  bool pick = ctx.fast_fft;
   try {
-    // 1. H*psi plane kernel: register-lane shapes (FP32 lengths with a
-    // register plan), then the warp-per-line kernel
-    {
-      std::vector<std::pair<int, int>> cand;   // (lane shape, warp shape)
-      if (ctx.precision == MIXED) {
-        for (int s : {4, 0, 3, 5, 6}) cand.push_back({s, ctx.fast_vpsi_shape});
-        for (int s : {0, 1}) cand.push_back({-1, s});
-      } else {
-        cand.push_back({-1, ctx.fast_vpsi_shape});
+    QBX_CUDA(cudaEventCreate(&e0));
+    QBX_CUDA(cudaEventCreate(&e1));
+    for (int f = line ? 1 : 0; f >= 0; f--) {
+      if (line) ctx.fast_fft = f == 1;
+      double t = 0.0;
+      for (int rep = 0; rep < 2; rep++) {   // the first pass warms up
+        QBX_CUDA(cudaEventRecord(e0, ctx.stream));
+        launch_vpsi(ctx, ctx.d_c, ctx.d_vr, ctx.d_ctmp);
+        launch_density(ctx, ctx.d_c, rho_tmp);
+        QBX_CUDA(cudaEventRecord(e1, ctx.stream));
+        QBX_CUDA(cudaEventSynchronize(e1));
+        float ms = 0.f;
+        QBX_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+        t = ms;
       }
-      double best = 1e30;
-      std::pair<int, int> pick = cand[0];
-      for (auto cv : cand) {
-        ctx.fast_lane_shape = cv.first;
-        ctx.fast_vpsi_shape = cv.second;
-        const double t = time_ms(vpsi);
-        note("vpsi lane " + std::to_string(cv.first) + " warp " + std::to_string(cv.second), t);
-        if (t < best) { best = t; pick = cv; }
-      }
-      ctx.fast_lane_shape = pick.first;
-      ctx.fast_vpsi_shape = pick.second;
-    }
-    // 2. density plane kernel shape
-    if (ctx.precision == MIXED && ctx.fast_lane_shape >= 0) {
-      double best = 1e30;
-      int pick = ctx.fast_density_lane_shape;
-      for (int s : {3, 2, 5, 6, 7, 8}) {
-        ctx.fast_density_lane_shape = s;
-        const double t = time_ms(dens);
-        note("density lane " + std::to_string(s), t);
-        if (t < best) { best = t; pick = s; }
-      }
-      ctx.fast_density_lane_shape = pick;
-      // CTAs per plane (each accumulates its share of the band pairs)
-      int pick_c = ctx.fast_chunks;
-      for (int ch : {4, 8, 12, 16}) {
-        ctx.fast_chunks = ch;
-        const double t = time_ms(dens);
-        note("density CTAs per plane " + std::to_string(ch), t);
-        if (t < best) { best = t; pick_c = ch; }
-      }
-      ctx.fast_chunks = pick_c;
-    }
-    // 3. band pairs per launch (the stick buffer stays in L2 for small batches)
-    {
-      const size_t per_pair = (ctx.precision == MIXED ? sizeof(float2) : sizeof(double2)) *
-                              (size_t)ctx.dws.n2 * ctx.dws.nvec;
-      const int cap = (int)std::max<size_t>(1, ctx.zfast_bytes / per_pair);
-      double best = 1e30;
-      int pick = ctx.fast_batch;
-      for (int b : {16, 32, 64, 0}) {
-        if (b > cap) continue;
-        ctx.fast_batch = b;
-        const double t = time_ms(vpsi) + time_ms(dens);
-        note("pairs per launch " + std::to_string(b == 0 ? cap : b), t);
-        if (t < best) { best = t; pick = b; }
-      }
-      ctx.fast_batch = pick;
-    }
-    // 4. z-stick kernels (register lanes or a warp per stick) and rods per CTA
-    {
-      double best = 1e30;
-      int pick = ctx.fast_rods, pick_z = ctx.fast_zlane;
-      for (int zl : {1, 0}) {
-        if (zl == 0 && ctx.precision != MIXED) continue;
-        if (ctx.precision == MIXED) ctx.fast_zlane = zl;
-        for (int r : {8, 16, 24, 32}) {
-          ctx.fast_rods = r;
-          const double t = time_ms(vpsi);
-          note("z lanes " + std::to_string(ctx.fast_zlane) + " rods per z CTA " + std::to_string(r), t);
-          if (t < best) { best = t; pick = r; pick_z = ctx.fast_zlane; }
-        }
-      }
-      ctx.fast_rods = pick;
-      ctx.fast_zlane = pick_z;
+      if (log) log->push_back({f ? "line passes" : "runtime-radix kernels", t});
+      if (t < best) { best = t; pick = ctx.fast_fft; }
     }
   } catch (...) {
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    dfree(rho_tmp);
+    release();
     throw;
   }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  dfree(rho_tmp);
+  ctx.fast_fft = pick;
+  release();
+  return line && pick ? "line passes" : "runtime-radix kernels";
 }
 
 }  // namespace qbx

@@ -1,23 +1,7 @@
-// Register-resident 1-D FFTs split over a small group of lanes, for the FP32
-// plane pass (fft_fast.cuh).
-//
-// A line of N = T * M points is held by T consecutive lanes (T = 2 or 4),
-// M values per lane.  With the input index x = t + T k (lane t, register k)
-// the transform is
-//
-//   X[k2 + M m] = sum_t W_N^{t k2} W_T^{t m} ( sum_k x[t + T k] W_M^{k k2} )
-//
-// i.e. an M-point DFT in each lane's registers, a twiddle by W_N^{t k2}, and
-// T-point DFTs across the lanes of the group done with warp shuffles.  The
-// cross-lane DFT leaves output m = bitrev(t) on lane t; the opposite
-// direction starts from that distribution (decimation in time) and ends in
-// the natural one, so a backward transform, a pointwise operation and a
-// forward transform need no reordering.  No shared memory is used for the
-// line itself and no warp synchronisation other than the shuffles.
-//
-// The M-point register DFT is a compile-time mixed-radix Cooley-Tukey
-// recursion (radices 2, 3, 4, 5, 7, 11 of fft_reg.cuh); its twiddles are
-// compile-time constants computed by a constexpr cosine/sine below.
+// Register DFTs of composite length for the FFT kernels (fft_pencil.cuh): a
+// compile-time mixed-radix Cooley-Tukey recursion over the short DFTs of
+// fft_reg.cuh, its twiddles compile-time constants computed by a constexpr
+// cosine/sine below.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -141,119 +125,6 @@ __device__ __forceinline__ void dft_reg(C (&v)[M]) {
       for (int s2 = 0; s2 < R; ++s2) v[q + Q * s2] = w[s2];
     }
   }
-}
-
-// ------------------------------------------------------------ lane groups
-template <typename C> __device__ __forceinline__ C shfl_xor(C v, int m) {
-  C r;
-  r.x = __shfl_xor_sync(0xffffffffu, v.x, m);
-  r.y = __shfl_xor_sync(0xffffffffu, v.y, m);
-  return r;
-}
-
-__host__ __device__ constexpr int bitrev(int t, int T) {
-  int r = 0;
-  for (int b = 1; b < T; b <<= 1) {
-    r = (r << 1) | (t & 1);
-    t >>= 1;
-  }
-  return r;
-}
-
-// One butterfly of a cross-lane stage: the lower lane of the pair keeps
-// a + b, the upper one b - a, both as s*a + b with s = +-1 per lane (an
-// exact fused multiply-add), so every lane runs the same two instructions
-// instead of forming both results and selecting one.
-template <typename C> __device__ __forceinline__ C lane_bfly(C a, C b, float s) {
-  using Real = decltype(a.x);
-  C r;
-  r.x = (Real)s * a.x + b.x;
-  r.y = (Real)s * a.y + b.y;
-  return r;
-}
-// x or x * (DIR i), chosen per lane
-template <int DIR, typename C> __device__ __forceinline__ C rot_if(C x, bool rot) {
-  const C r = reg::cmuli<DIR>(x);
-  C o;
-  o.x = rot ? r.x : x.x;
-  o.y = rot ? r.y : x.y;
-  return o;
-}
-
-// T-point DFT across the lanes t = 0..T-1 of a group, one value per lane:
-// natural input, output X[bitrev(t)] on lane t (decimation in frequency).
-template <int T, int DIR, typename C>
-__device__ __forceinline__ C group_dft_n2r(C a, int t) {
-  static_assert(T == 1 || T == 2 || T == 4, "lane groups of 1, 2 or 4");
-#pragma unroll
-  for (int h = T / 2; h >= 1; h >>= 1) {
-    const C b = shfl_xor(a, h);
-    const int j = t & (2 * h - 1);
-    a = lane_bfly(a, b, j < h ? 1.f : -1.f);
-    // W_{2h}^{j-h} on the upper lanes: only W_4^1 = DIR i is not 1
-    if (h == 2) a = rot_if<DIR>(a, j == 3);
-  }
-  return a;
-}
-
-// T-point DFT across the lanes of a group from the bit-reversed
-// distribution (lane t holds input bitrev(t)) to natural output
-// (decimation in time).
-template <int T, int DIR, typename C>
-__device__ __forceinline__ C group_dft_r2n(C a, int t) {
-#pragma unroll
-  for (int h = 1; h <= T / 2; h <<= 1) {
-    const int j = t & (2 * h - 1);
-    // the upper element of each butterfly is twiddled before the exchange
-    if (h == 2) a = rot_if<DIR>(a, j == 3);
-    const C b = shfl_xor(a, h);
-    a = lane_bfly(a, b, j < h ? 1.f : -1.f);
-  }
-  return a;
-}
-
-// ------------------------------------------------------------ whole lines
-// Line of N = T M points, lane t of the group holds v[k] = x[t + T k].
-// Backward-style transform (direction DIR) leaving v[k2] = X[k2 + M bitrev(t)].
-template <int T, int M, int DIR, typename C>
-__device__ __forceinline__ void line_n2r(C (&v)[M], int t, const C* tw /* N entries */) {
-  dft_reg<M, DIR>(v);
-  if constexpr (T > 1) {
-    // twiddle loads stay after the register DFT (hoisted above it they would
-    // hold M more values in registers through it)
-    asm volatile("" ::: "memory");
-#pragma unroll
-    for (int k2 = 1; k2 < M; ++k2) {
-      const C w = tw[t * k2];
-      v[k2] = DIR > 0 ? cmul(v[k2], w) : cmulc(v[k2], w);
-    }
-#pragma unroll
-    for (int k2 = 0; k2 < M; ++k2) v[k2] = group_dft_n2r<T, DIR>(v[k2], t);
-  }
-}
-
-// The opposite: lane t holds v[k2] = x[k2 + M bitrev(t)]; afterwards
-// v[k] = X[t + T k].
-template <int T, int M, int DIR, typename C>
-__device__ __forceinline__ void line_r2n(C (&v)[M], int t, const C* tw) {
-  if constexpr (T > 1) {
-#pragma unroll
-    for (int k2 = 0; k2 < M; ++k2) v[k2] = group_dft_r2n<T, DIR>(v[k2], t);
-    asm volatile("" ::: "memory");
-#pragma unroll
-    for (int k2 = 1; k2 < M; ++k2) {
-      const C w = tw[t * k2];
-      v[k2] = DIR > 0 ? cmul(v[k2], w) : cmulc(v[k2], w);
-    }
-  }
-  dft_reg<M, DIR>(v);
-}
-
-// Lanes per line for a length: 4 when N/4 has a register plan of at most 36
-// points, else 2 (N/2 <= 36), else 0 (no register plan).
-__host__ __device__ constexpr int lanes_for(int n) {
-  return (n % 4 == 0 && n / 4 <= 36 && reg_ok(n / 4)) ? 4
-       : (n % 2 == 0 && n / 2 <= 36 && reg_ok(n / 2)) ? 2 : 0;
 }
 
 }  // namespace lane

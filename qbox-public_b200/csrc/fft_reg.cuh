@@ -1,30 +1,12 @@
-// Warp-synchronous 1-D FFTs of compile-time length for the staged 3-D
-// transforms (fft_fast.cuh).
-//
-// One warp transforms one line of N complex values held in shared memory.
-// The length is factored into radix stages at compile time, odd radices
-// first (11, 7, 5, 3), then a 2, then 4s, so that the last stages write
-// stride-1 across the lanes.  Each stage is a self-sorting Stockham pass done
-// in place: every lane first loads the inputs of its butterflies (N/R of
-// them, spread over the 32 lanes) into registers, the warp synchronises, and
-// the lanes then twiddle, transform and store.  Only __syncwarp separates the
-// stages, so the warps of a CTA work on different lines independently.
-//
-// The first stage can read its inputs through a loader functor and the last
-// stage can hand its outputs to a storer functor, which is how the kernels
-// fuse the gather from the coefficient sphere or the plane tile, the
-// multiplication by V(r) and the density accumulation into the transforms.
+// Complex arithmetic and the short prime DFTs in registers (2, 3, 4, 5, 7,
+// 11 points) that the register transforms of fft_lane.cuh are built from.
 //
 // Sign convention: DIR = +1 computes out[k] = sum_j in[j] exp(+2 pi i jk/N)
 // (the reference's backward transform, unscaled), DIR = -1 the forward one.
-// Twiddles exp(+2 pi i k/N) come from a length-N table in shared memory,
-// conjugated for DIR = -1.  The small DFTs use the cosines and sines of
-// 2 pi j/R as literal constants.
+// The small DFTs use the cosines and sines of 2 pi j/R as literal constants.
 #pragma once
 
 #include <cuda_runtime.h>
-
-#include <cstdint>
 
 namespace qbx {
 namespace reg {
@@ -32,34 +14,6 @@ namespace reg {
 template <typename T> struct CT;
 template <> struct CT<float> { using c = float2; };
 template <> struct CT<double> { using c = double2; };
-
-// ------------------------------------------------------------ plan
-struct CPlan {
-  int n = 0, ns = 0, rest = 1;
-  int r[16] = {0};
-};
-
-__host__ __device__ constexpr CPlan cplan(int n) {
-  CPlan p{};
-  p.n = n;
-  int m = n, twos = 0;
-  while (m % 2 == 0) { m /= 2; ++twos; }
-  const int odd[4] = {11, 7, 5, 3};
-  for (int i = 0; i < 4; ++i)
-    while (m % odd[i] == 0) { p.r[p.ns++] = odd[i]; m /= odd[i]; }
-  if (twos % 2) p.r[p.ns++] = 2;
-  for (int i = 0; i < twos / 2; ++i) p.r[p.ns++] = 4;
-  p.rest = m;
-  return p;
-}
-__host__ __device__ constexpr int stage_count(int n) { return cplan(n).ns; }
-__host__ __device__ constexpr int stage_radix(int n, int s) { return cplan(n).r[s]; }
-__host__ __device__ constexpr int stage_ns(int n, int s) {
-  int p = 1;
-  for (int i = 0; i < s; ++i) p *= cplan(n).r[i];
-  return p;
-}
-__host__ __device__ constexpr bool plan_ok(int n) { return n > 1 && cplan(n).rest == 1; }
 
 // cos(2 pi j/R), sin(2 pi j/R) for 1 <= j <= (R-1)/2
 __host__ __device__ constexpr double rcos(int R, int j) {
@@ -150,141 +104,6 @@ __device__ __forceinline__ void dft(C (&v)[R]) {
 #pragma unroll
     for (int k = 0; k < R; ++k) v[k] = out[k];
   }
-}
-
-// ------------------------------------------------------------ functors
-template <typename C> struct BufLoad {
-  const C* b;
-  __device__ __forceinline__ C operator()(int i) const { return b[i]; }
-};
-template <typename C> struct BufStore {
-  C* b;
-  __device__ __forceinline__ void operator()(int i, C v) const { b[i] = v; }
-};
-
-// ------------------------------------------------------------ shared memory
-// The working line and the twiddle table are addressed through 32-bit
-// shared-window offsets that the optimiser cannot see through (see
-// warp_fft), with explicit ld/st.shared.
-__device__ __forceinline__ float2 lds(uint32_t a, float2*) {
-  float2 v;
-  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ double2 lds(uint32_t a, double2*) {
-  double2 v;
-  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ void sts(uint32_t a, float2 v) {
-  asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
-}
-__device__ __forceinline__ void sts(uint32_t a, double2 v) {
-  asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
-}
-__device__ __forceinline__ void warp_sync_mem() {
-  asm volatile("" ::: "memory");
-  __syncwarp();
-  asm volatile("" ::: "memory");
-}
-
-// ------------------------------------------------------------ stages
-// First-stage geometry of a length-N line: lane + 32*rd is the butterfly,
-// q its input; input index = butterfly + q * NB.
-template <int N> struct FirstStage {
-  static constexpr int R = stage_radix(N, 0);
-  static constexpr int NB = N / R;
-  static constexpr int RD = (NB + 31) / 32;
-};
-
-template <int N, int S, int DIR, typename C, typename LD, typename ST>
-__device__ __forceinline__ void wstage(uint32_t sbuf, uint32_t stw, int lane, const LD& ld,
-                                       const ST& st) {
-  constexpr int R = stage_radix(N, S);
-  constexpr int NS = stage_ns(N, S);
-  constexpr int NB = N / R;
-  constexpr int RD = (NB + 31) / 32;
-  constexpr bool FIRST = (S == 0);
-  constexpr bool LAST = (S == stage_count(N) - 1);
-  constexpr uint32_t E = sizeof(C);
-  C v[RD][R];
-#pragma unroll
-  for (int rd = 0; rd < RD; ++rd) {
-    const int i = lane + 32 * rd;
-    if (NB % 32 == 0 || i < NB) {
-#pragma unroll
-      for (int q = 0; q < R; ++q) {
-        if constexpr (FIRST) v[rd][q] = ld(rd, q, i + q * NB);
-        else v[rd][q] = lds(sbuf + (uint32_t)(i + q * NB) * E, (C*)nullptr);
-      }
-    }
-  }
-  warp_sync_mem();
-#pragma unroll
-  for (int rd = 0; rd < RD; ++rd) {
-    const int i = lane + 32 * rd;
-    if (NB % 32 == 0 || i < NB) {
-      const int j = i % NS;
-      if constexpr (NS > 1) {
-        constexpr int TS = N / (NS * R);
-#pragma unroll
-        for (int q = 1; q < R; ++q) {
-          const C w = lds(stw + (uint32_t)(q * j * TS) * E, (C*)nullptr);
-          v[rd][q] = DIR > 0 ? cmul(v[rd][q], w) : cmulc(v[rd][q], w);
-        }
-      }
-      dft<R, DIR>(v[rd]);
-      const int base = (i - j) * R + j;
-#pragma unroll
-      for (int q = 0; q < R; ++q) {
-        if constexpr (LAST) st(base + q * NS, v[rd][q]);
-        else sts(sbuf + (uint32_t)(base + q * NS) * E, v[rd][q]);
-      }
-    }
-  }
-  warp_sync_mem();
-}
-
-template <int N, int S, int DIR, typename C, typename LD, typename ST>
-__device__ __forceinline__ void wstages(uint32_t sbuf, uint32_t stw, int lane, const LD& ld,
-                                        const ST& st) {
-  wstage<N, S, DIR, C>(sbuf, stw, lane, ld, st);
-  if constexpr (S + 1 < stage_count(N)) wstages<N, S + 1, DIR, C>(sbuf, stw, lane, ld, st);
-}
-
-// Adapts a loader of the form ld(i) to the first stage's ld(rd, q, i).
-template <typename LD> struct IndexLoad {
-  const LD& f;
-  __device__ __forceinline__ auto operator()(int, int, int i) const { return f(i); }
-};
-
-// Transform one line with the warp.  buf (N values, shared memory) is the
-// working line; ld(i) supplies input i to the first stage, st(k, value)
-// takes output k from the last stage.
-template <int N, int DIR, typename C, typename LD, typename ST>
-__device__ __forceinline__ void warp_fft(C* buf, const C* tw, int lane, const LD& ld, const ST& st) {
-  static_assert(plan_ok(N), "FFT length must factor into 2, 3, 5, 7, 11");
-  uint32_t sbuf = (uint32_t)__cvta_generic_to_shared(buf);
-  uint32_t stw = (uint32_t)__cvta_generic_to_shared(tw);
-  // Hide the addresses and the lane from the optimiser: otherwise it keeps
-  // every lane's twiddle and line offsets of every stage in registers across
-  // the callers' loops, which costs more registers (and occupancy) than
-  // recomputing them.
-  asm volatile("" : "+r"(sbuf), "+r"(stw), "+r"(lane));
-  wstages<N, 0, DIR, C>(sbuf, stw, lane, IndexLoad<LD>{ld}, st);
-}
-
-// As warp_fft, with a first-stage loader that also receives the butterfly
-// round rd and input q (for values the caller prefetched into registers in
-// FirstStage<N> order).
-template <int N, int DIR, typename C, typename LD, typename ST>
-__device__ __forceinline__ void warp_fft_rq(C* buf, const C* tw, int lane, const LD& ld,
-                                            const ST& st) {
-  static_assert(plan_ok(N), "FFT length must factor into 2, 3, 5, 7, 11");
-  uint32_t sbuf = (uint32_t)__cvta_generic_to_shared(buf);
-  uint32_t stw = (uint32_t)__cvta_generic_to_shared(tw);
-  asm volatile("" : "+r"(sbuf), "+r"(stw), "+r"(lane));
-  wstages<N, 0, DIR, C>(sbuf, stw, lane, ld, st);
 }
 
 }  // namespace reg

@@ -128,6 +128,7 @@ struct DeviceSticks {
   int* stick_y;      // nvec
   int* stick_col;    // nvec
   int* col_x;        // ncol
+  int* xcol;         // n0: the compact column at x, -1 if none
   int* ip;           // ng
   int* im;           // ng
   RadixPlan px, py, pz;
@@ -135,12 +136,13 @@ struct DeviceSticks {
                      // so contexts of different grids never share tables)
   int* colmap;       // ncol x n1: the stick at (compact column, y), -1 if none
   // widest occupied distance from 0 (mod n) of the stick columns' x, the
-  // sticks' y and the rods' z: the pruned plane and z kernels skip the lane
-  // registers that only hold points beyond prune_width(n)
+  // sticks' y and the rods' z: the line kernels load and store only the
+  // points that lie within prune_width(n)
   int xw, yw, zw;
+  double gain32;     // pencil_gain_fp32 of the three lengths, multiplied
 };
 
-// Points of a line of length n that the pruned kernels keep: x with
+// Points of a line of length n that the line kernels keep: x with
 // min(x, n - x) <= prune_width(n).  A wavefunction basis on the grid Qbox
 // builds for its density (n >= 4 hmax + 1) always fits.
 __host__ __device__ constexpr int prune_width(int n) { return (n - 1) / 4; }
@@ -294,6 +296,7 @@ struct KPointSet {
   double* d_w2 = nullptr;      // weight*occ/Omega twice per band (plane kernel weights)
   double* d_prec = nullptr;    // nst per-band kinetic energies
   bool anl_ready = false;
+  bool tile_valid = false;     // its tiles are those of its current coefficients
   double theta = 0;
 };
 
@@ -455,23 +458,7 @@ struct Context {
   float* d_vr32 = nullptr;      // FP32 copy of V(r) for the mixed H*psi pass
   void* d_zfast = nullptr;      // stick buffer of the specialised staged FFTs
   size_t zfast_bytes = 0;
-  int fast_batch = 0;           // band pairs per launch (0: as many as fit)
-  int fast_rods = 16;           // rods per CTA of the z kernels
-  int fast_warps = 16;          // warps per CTA of the plane kernel (at most)
-  int fast_vpsi_shape = 0;      // FP32 H*psi plane CTA shape (0, 1, 2)
-  int fast_lane_shape = 4;      // FP32 register-lane plane kernel shape (5: sticks through
-                                // the column map), -1 = off
-  int fast_density_lane_shape = 3;  // its density shape (2, 3; 5 half planes; 6 sticks
-                                    // read through the column map; 7 TMEM accumulator;
-                                    // 8 next pair's sticks queued with cp.async)
-  int fast_chunks = 8;          // CTAs per plane in the density pass
-  int fast_fwd_ppc = 2;         // band pairs per CTA of the H*psi plane kernel from psi(r)
-  int fast_fwd_staged = 1;      // that kernel with its rows staged by cp.async
-  int fast_prune = 1;           // FP32 lane kernels skip the points beyond the sphere
-                                // (prune_width) where the basis allows it
-  int fast_zlane = 1;           // FP32 z sticks in register lanes (0: warp per stick;
-                                // 2: backward uncapped; 3: forward only)
-  bool fast_fft = true;         // use the specialised kernels when compiled
+  bool fast_fft = true;         // the line-pass FFTs (fft_pencil.cuh) where they take the grid
   float* a32 = nullptr;         // TF32 hi/lo split of the projectors
   float* a32lo = nullptr;
   float* s32 = nullptr;         // TF32 hi/lo split of a small matrix
@@ -506,14 +493,15 @@ struct Context {
   long batch_launches = 0;       // batch graphs launched with this context leading
   int polar_iters = 0;           // iterations of the last eager polar
   double* d_wfv = nullptr;       // wavefunction velocity of the MD extrapolation
-  // psi(r) of every band pair kept in HBM (FP32) from the density pass to
-  // the H*psi pass of the same step: the step functions set psir_store
-  // around update_density and psir_use around energy
-  float2* d_psir = nullptr;
-  size_t psir_bytes = 0;
-  int psir_mode = -1;            // -1 auto (mixed precision, if it fits), 0 off, 1 on
-  bool psir_store = false, psir_use = false, psir_valid = false;
-  const double* psir_src = nullptr;   // the coefficients psi(r) was made from
+  // the y-transformed tiles of every band pair (or band of every k point)
+  // kept in HBM from the density pass to the H*psi pass of the same step, which
+  // then starts at the x transform: the step functions set tile_store around
+  // update_density and tile_use around energy
+  void* d_wtile = nullptr;
+  size_t wtile_bytes = 0;
+  int wtile_mode = -1;           // -1 where it fits, 0 off, 1 on
+  bool tile_store = false, tile_use = false, tile_valid = false;
+  const double* tile_src = nullptr;   // the coefficients the tiles were made from
   // streamed SlaterDet (qbx_stream_in / qbx_scf_step_async / qbx_stream_out):
   // two copy streams, the staging buffers of one step's input and result,
   // and the events that order them against the compute stream
@@ -608,7 +596,7 @@ void vb_forward_real_pair(Context& ctx, const double* f0, const double* f1, cons
 void wb_backward_pair(Context& ctx, const double* c1, const double* c2, double* grid_out);
 
 // staged-FFT launch configuration by timing on the context's own data
-void autotune_fft(Context& ctx, std::vector<std::pair<std::string, double>>* log);
+std::string autotune_fft(Context& ctx, std::vector<std::pair<std::string, double>>* log);
 
 // occ_n / Omega per band (device), used by the density kernels
 double* density_weights(Context& ctx);

@@ -173,7 +173,7 @@ int qbx_set_band_shard(qbx_context* h, int rank, int nranks,
       c.shard_rank = rank;
       c.shard_n = nranks;
     }
-    c.psir_valid = false;
+    c.tile_valid = false;
     c.last_error.clear();
     return 0;
   } catch (const qbx::Error& e) {
