@@ -147,6 +147,14 @@ void check_ready(const Context& c, bool atoms) {
 
 }  // namespace
 
+// the caller's x-fastest form of one of the context's grids: f itself or its
+// transpose in the scratch grid
+static double* caller_grid(Context& c, double* f) {
+  if (!c.grid_zfast) return f;
+  grid_to_caller(c, f, (double*)c.d_grid);
+  return (double*)c.d_grid;
+}
+
 // density weights live after the scalar slots
 namespace qbx {
 double* density_weights(Context& c) { return c.d_scalars + kSlots; }
@@ -555,6 +563,7 @@ int qbx_set_cell(qbx_context* h, const double cell[9], double ecut, int nst, con
     }
     c.species.clear();
     c.tau.clear();
+    c.grid_zfast = grid_zfast_possible(c);
     QBX_CUDA(cudaDeviceSynchronize());   // memsets above ran on the legacy stream
     c.have_cell = true;
     alloc_mixed(c);
@@ -926,7 +935,8 @@ int qbx_update_density(qbx_context* h, double* total_charge) {
 int qbx_get_density(qbx_context* h, double* rhor) {
   return guarded(h, [&](Context& c) {
     check_ready(c, false);
-    QBX_CUDA(cudaMemcpyAsync(rhor, c.d_rhor, c.N() * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    QBX_CUDA(cudaMemcpyAsync(rhor, caller_grid(c, c.d_rhor), c.N() * sizeof(double),
+                             cudaMemcpyDeviceToHost, c.stream));
     QBX_CUDA(cudaStreamSynchronize(c.stream));
   });
 }
@@ -943,7 +953,8 @@ int qbx_update_vhxc(qbx_context* h) {
 int qbx_get_vr(qbx_context* h, double* vr) {
   return guarded(h, [&](Context& c) {
     check_ready(c, false);
-    QBX_CUDA(cudaMemcpyAsync(vr, c.d_vr, c.N() * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    QBX_CUDA(cudaMemcpyAsync(vr, caller_grid(c, c.d_vr), c.N() * sizeof(double),
+                             cudaMemcpyDeviceToHost, c.stream));
     QBX_CUDA(cudaStreamSynchronize(c.stream));
   });
 }
@@ -1421,8 +1432,8 @@ int qbx_compute_density(qbx_context* h, double weight, double* rho) {
     if (!c.d_xgrid) c.d_xgrid = dalloc<double>(N);
     launch_density(c, c.d_c, c.d_xgrid);
     std::vector<double> tmp(N);
-    QBX_CUDA(cudaMemcpyAsync(tmp.data(), c.d_xgrid, N * sizeof(double), cudaMemcpyDeviceToHost,
-                             c.stream));
+    QBX_CUDA(cudaMemcpyAsync(tmp.data(), caller_grid(c, c.d_xgrid), N * sizeof(double),
+                             cudaMemcpyDeviceToHost, c.stream));
     QBX_CUDA(cudaStreamSynchronize(c.stream));
     for (size_t i = 0; i < N; i++) rho[i] += weight * tmp[i];
   });
@@ -1436,7 +1447,9 @@ int qbx_rs_mul_add(qbx_context* h, const double* v, double* dc) {
     const size_t N = c.N();
     if (!c.d_xgrid) c.d_xgrid = dalloc<double>(N);
     double* out = lazy_wf(c, c.d_xsd);
-    QBX_CUDA(cudaMemcpyAsync(c.d_xgrid, v, N * sizeof(double), cudaMemcpyHostToDevice, c.stream));
+    double* in = c.grid_zfast ? (double*)c.d_grid : c.d_xgrid;
+    QBX_CUDA(cudaMemcpyAsync(in, v, N * sizeof(double), cudaMemcpyHostToDevice, c.stream));
+    if (c.grid_zfast) grid_from_caller(c, in, c.d_xgrid);
     launch_vpsi(c, c.d_c, c.d_xgrid, out);   // 1/2 G^2 c + V psi
     k_sub_kinetic<<<1184, 256, 0, c.stream>>>((double2*)out, (const double2*)c.d_c, c.d_g2_w,
                                               c.wb.ng, c.nst);

@@ -750,6 +750,56 @@ k_grid_to_zfast(const A* __restrict__ in, int n0, int n1, int n2, bool to_zfast,
   }
 }
 
+static int nblk(size_t n);
+static bool pencil_ok(const Context& ctx, const DeviceSticks& g, bool fp32);
+
+__global__ void k_to_float(const double* __restrict__ x, size_t n, float* __restrict__ y) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x)
+    y[i] = (float)x[i];
+}
+
+// The context's real-space grids (density, potentials, gradients) are kept z
+// fastest when both of its bases go through the line passes, which then read
+// and write them directly; callers of the library always see x fastest.
+bool grid_zfast_possible(const Context& ctx) {
+  const DeviceSticks& g = ctx.dvs;
+  return pencil_ok(ctx, ctx.dws, false) && ctx.zfast_bytes >=
+         sizeof(double2) * (size_t)g.n2 * ((size_t)g.nvec + (size_t)g.ncol * g.n1);
+}
+
+// f as callers see it (x fastest), in `out`; and the opposite
+void grid_to_caller(Context& ctx, const double* f, double* out) {
+  const DeviceSticks& g = ctx.dvs;
+  const dim3 tg((g.n0 + 31) / 32, (g.n2 + 31) / 32, g.n1);
+  k_grid_to_zfast<double, double, false><<<tg, 256, 0, ctx.stream>>>(f, g.n0, g.n1, g.n2, false,
+                                                                     out);
+  QBX_LAUNCHED(ctx);
+}
+void grid_from_caller(Context& ctx, const double* f, double* out) {
+  const DeviceSticks& g = ctx.dvs;
+  const dim3 tg((g.n0 + 31) / 32, (g.n2 + 31) / 32, g.n1);
+  k_grid_to_zfast<double, double, false><<<tg, 256, 0, ctx.stream>>>(f, g.n0, g.n1, g.n2, true,
+                                                                     out);
+  QBX_LAUNCHED(ctx);
+}
+
+// With k points the grids are z fastest only if every k point's sphere runs
+// through the line passes; the density and potential that the context holds
+// move to the new order.
+void kpoints_grid_order(Context& ctx) {
+  bool z = grid_zfast_possible(ctx);
+  for (const KPointSet& kp : ctx.kpts) z = z && pencil_ok(ctx, kp.dks, false);
+  if (z == ctx.grid_zfast) return;
+  for (double* f : {ctx.d_rhor, ctx.d_vr}) {
+    if (z) grid_from_caller(ctx, f, (double*)ctx.d_grid);
+    else grid_to_caller(ctx, f, (double*)ctx.d_grid);
+    QBX_CUDA(cudaMemcpyAsync(f, ctx.d_grid, ctx.N() * sizeof(double), cudaMemcpyDeviceToDevice,
+                             ctx.stream));
+  }
+  ctx.grid_zfast = z;
+}
+
 template <typename T>
 static bool pencil_run(Context& ctx, int n, const pen::Args& a) {
   return pencil_0<T>(ctx, n, a) || pencil_1<T>(ctx, n, a) || pencil_2<T>(ctx, n, a) ||
@@ -872,13 +922,22 @@ static void pencil_pass(Context& ctx, const DeviceSticks& g, bool complex_basis,
   a.nst = ctx.nst;
   a.w = w;
   a.nw = nw;
-  a.rho = (double*)ctx.d_grid;              // density and V(r), z fastest
+  // density and V(r), z fastest: the context's own grids where they are kept
+  // so (grid_zfast), else transposed through d_grid
+  const bool zfast = ctx.grid_zfast;
+  a.rho = zfast ? rho : (double*)ctx.d_grid;
   T* vt = (T*)((double*)ctx.d_grid + N);
   a.v = vt;
   a.stream = ctx.stream;
   if (op == OP_VPSI) {
-    k_grid_to_zfast<double, T, false><<<tg, 256, 0, ctx.stream>>>(v, g.n0, g.n1, g.n2, true, vt);
-    QBX_LAUNCHED(ctx);
+    if (zfast && sizeof(T) == 8) {
+      a.v = v;
+    } else {
+      if (zfast) k_to_float<<<nblk(N), 256, 0, ctx.stream>>>(v, N, (float*)vt);
+      else k_grid_to_zfast<double, T, false><<<tg, 256, 0, ctx.stream>>>(v, g.n0, g.n1, g.n2, true,
+                                                                        vt);
+      QBX_LAUNCHED(ctx);
+    }
   }
   const size_t sb = pencil_stick_bytes(g, sizeof(T) == 4), tb = pencil_tile_bytes(g, sizeof(T) == 4);
   const int batch = (int)std::min<size_t>(nslots, ctx.zfast_bytes / (area ? sb : sb + tb));
@@ -916,8 +975,8 @@ static void pencil_pass(Context& ctx, const DeviceSticks& g, bool complex_basis,
     slots(s0, ns);
     const int ch = chunks(ns, xcta, 16);
     if (op == OP_DENSITY) {
-      a.rho_set = s0 == 0 && ch == 1;
-      if (s0 == 0 && !a.rho_set)
+      a.rho_set = s0 == 0 && ch == 1 && !(zfast && add);
+      if (s0 == 0 && !a.rho_set && !(zfast && add))
         QBX_CUDA(cudaMemsetAsync(a.rho, 0, N * sizeof(double), ctx.stream));
       pass(g.n0, pen::XD, ch, "xy_density");
     } else {
@@ -936,7 +995,7 @@ static void pencil_pass(Context& ctx, const DeviceSticks& g, bool complex_basis,
     for (int s0 = 0; op == OP_VPSI && s0 < nslots; s0 += batch)
       forth(s0, std::min(batch, nslots - s0));
   }
-  if (op == OP_DENSITY) {
+  if (op == OP_DENSITY && !zfast) {
     if (add)
       k_grid_to_zfast<double, double, true><<<tg, 256, 0, ctx.stream>>>(a.rho, g.n0, g.n1, g.n2,
                                                                         false, rho);
@@ -976,6 +1035,7 @@ static void staged_k(Context& ctx, KPointSet& kp, int op, const double* v, doubl
     kp.tile_valid = op == OP_DENSITY && area && ctx.tile_store;
     return;
   }
+  QBX_REQUIRE(!ctx.grid_zfast, 21, "this k point's sphere does not fit the line passes");
   cudaStream_t st = ctx.stream;
   double2* zbuf = (double2*)ctx.d_zbuf;
   const int ngw = kp.kb.ng;
@@ -1169,6 +1229,13 @@ void wfgrid_forward(Context& ctx, const DeviceSticks& d, int ng, const double* f
 
 static int nblk(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 148 * 16); }
 
+// z = x + y (z may be either)
+__global__ void k_add(const double* x, const double* y, size_t n, double* z) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x)
+    z[i] = x[i] + y[i];
+}
+
 // ----------------------------------------------- a caller's basis and grid
 // The grid of a FourierTransform built on any basis (its Miller indices in
 // the caller's order): sizes, twiddle tables, radix plans and the grid
@@ -1233,7 +1300,66 @@ void basis_ft_forward(Context& ctx, const DeviceSticks& d, int ng, bool real_bas
   QBX_LAUNCHED(ctx);
 }
 
+// ------------------------------------------- transforms of the density basis
+// One complex FP64 transform of one or two real fields between the density
+// sphere and the context's grids.  Kept z fastest, they run as the line
+// passes of fft_pencil.cuh on the density sphere's sticks: three kernels that
+// read the coefficients and write the fields, in place of a cleared grid, a
+// scatter, three in-place passes over the whole grid and an extraction.  With
+// the GGA's last two fields packed into one transform, update_vhxc takes (ms)
+// 0.45 -> 0.22 at 84^3 and 1.24 -> 0.57 at 140^3, PBE; what is left there is
+// the latency of some twenty short kernels, and at 140^3 HBM.
+static pen::Args field_args(Context& ctx) {
+  const DeviceSticks& g = ctx.dvs;
+  pen::Args a;
+  a.g = g;
+  for (int i = 0; i < 3; i++) a.tw[i] = g.tw[i];
+  a.scale = 1.0 / (double)ctx.N();
+  a.ngw = ctx.vb.ng;
+  a.nslots = 1;
+  a.sticks = ctx.d_zfast;
+  a.tile = (double2*)ctx.d_zfast + (size_t)g.nvec * g.n2;
+  a.stream = ctx.stream;
+  return a;
+}
+static void field_passes(Context& ctx, pen::Args& a, bool back) {
+  ProfScope ps(ctx, "grid_fft");
+  const DeviceSticks& g = ctx.dvs;
+  const int order[3] = {back ? pen::GZB : pen::GXG, back ? pen::GYB : pen::GYF,
+                        back ? pen::GXR : pen::GZF};
+  const int n[3] = {back ? g.n2 : g.n0, g.n1, back ? g.n0 : g.n2};
+  for (int i = 0; i < 3; i++) {
+    a.op = order[i];
+    QBX_REQUIRE(pencil_run<double>(ctx, n[i], a), 21, "no line kernel of this length");
+  }
+}
+// f0 = Re (+ add), f1 = Im (+ the new f0 with `chain`) of the transform of
+// c0 + i c1 (c1, f1 may be null)
+static void fields_backward(Context& ctx, const double* c0, const double* c1, double* f0,
+                            double* f1, const double* add, bool chain) {
+  pen::Args a = field_args(ctx);
+  a.c = (const double2*)c0;
+  a.cb = (const double2*)c1;
+  a.f0 = f0;
+  a.f1 = f1;
+  a.fadd = add;
+  a.chain = chain;
+  field_passes(ctx, a, true);
+}
+static void fields_forward(Context& ctx, const double* f0, const double* f1, const double* mul,
+                           double scale, double* c0, double* c1) {
+  pen::Args a = field_args(ctx);
+  a.f0 = (double*)f0;
+  a.f1 = (double*)f1;
+  a.fmul = mul;
+  a.scale *= scale;
+  a.hc = (double2*)c0;
+  a.hcb = (double2*)c1;
+  field_passes(ctx, a, false);
+}
+
 void vb_backward(Context& ctx, const double* coef, double* real_out) {
+  if (ctx.grid_zfast) return fields_backward(ctx, coef, nullptr, real_out, nullptr, nullptr, false);
   const size_t N = ctx.N();
   QBX_CUDA(cudaMemsetAsync(ctx.d_grid, 0, N * sizeof(double2), ctx.stream));
   k_scatter_sphere<<<nblk(ctx.vb.ng), 256, 0, ctx.stream>>>((const double2*)coef, ctx.dvs.ip,
@@ -1245,6 +1371,7 @@ void vb_backward(Context& ctx, const double* coef, double* real_out) {
 }
 
 void vb_backward_pair(Context& ctx, const double* a, const double* b, double* out0, double* out1) {
+  if (ctx.grid_zfast) return fields_backward(ctx, a, b, out0, out1, nullptr, false);
   const size_t N = ctx.N();
   QBX_CUDA(cudaMemsetAsync(ctx.d_grid, 0, N * sizeof(double2), ctx.stream));
   k_scatter_pair<<<nblk(ctx.vb.ng), 256, 0, ctx.stream>>>((const double2*)a, (const double2*)b,
@@ -1258,6 +1385,7 @@ void vb_backward_pair(Context& ctx, const double* a, const double* b, double* ou
 
 void vb_forward_real_pair(Context& ctx, const double* f0, const double* f1, const double* w,
                           double* c0, double* c1) {
+  if (ctx.grid_zfast) return fields_forward(ctx, f0, f1, w, 1.0, c0, c1);
   const size_t N = ctx.N();
   k_real2_mul_to_grid<<<nblk(N), 256, 0, ctx.stream>>>(f0, f1, w, N, (double2*)ctx.d_grid);
   QBX_LAUNCHED(ctx);
@@ -1275,12 +1403,28 @@ void vb_forward_real_pair(Context& ctx, const double* f0, const double* f1, cons
 }
 
 void vb_forward_real(Context& ctx, const double* f, double scale, double* coef) {
+  if (ctx.grid_zfast) return fields_forward(ctx, f, nullptr, nullptr, scale, coef, nullptr);
   const size_t N = ctx.N();
   k_real_to_grid<<<nblk(N), 256, 0, ctx.stream>>>(f, scale, N, (double2*)ctx.d_grid);
   QBX_LAUNCHED(ctx);
   grid_fft(ctx, -1);
   k_gather_sphere<<<nblk(ctx.vb.ng), 256, 0, ctx.stream>>>((const double2*)ctx.d_grid, ctx.dvs.ip,
                                                            ctx.vb.ng, 1.0 / (double)N, (double2*)coef);
+  QBX_LAUNCHED(ctx);
+}
+
+// out0 = add + back(a) and, with b, out1 = out0 + back(b): the sums over the
+// grid that follow a transform, in its last pass where the line passes run
+void vb_backward_add(Context& ctx, const double* a, const double* b, const double* add,
+                     double* out0, double* out1) {
+  if (ctx.grid_zfast) return fields_backward(ctx, a, b, out0, out1, add, b != nullptr);
+  const size_t N = ctx.N();
+  if (b) vb_backward_pair(ctx, a, b, (double*)ctx.d_exc, out1);
+  else vb_backward(ctx, a, ctx.d_exc);
+  k_add<<<nblk(N), 256, 0, ctx.stream>>>(add, ctx.d_exc, N, out0);
+  QBX_LAUNCHED(ctx);
+  if (!b) return;
+  k_add<<<nblk(N), 256, 0, ctx.stream>>>(out0, out1, N, out1);
   QBX_LAUNCHED(ctx);
 }
 
@@ -1356,49 +1500,42 @@ void density_with_buffers(Context& ctx, const double* c, int nst, const double* 
 namespace qbx {
 
 // ------------------------------------------------------------ autotuner
-// Picks the staged-FFT kernels for this context's grid, basis and precision
-// by timing the candidates on the context's own wavefunctions and potential:
-// the line passes (fft_pencil.cuh), where they take the grid, or the
-// runtime-radix kernels.  Returns the choice's name; the timings are
-// appended to `log`.
+// Times H psi and the density of this context's wavefunctions and names the
+// kernels that run them: the line passes (fft_pencil.cuh), whose shapes are
+// fixed per length at compile time, or the runtime-radix kernels on grids of
+// other lengths (the passes were the faster on every grid that has both).
+// The timings are appended to `log`.
 std::string autotune_fft(Context& ctx, std::vector<std::pair<std::string, double>>* log) {
   QBX_REQUIRE(ctx.have_cell && ctx.d_zfast, 7, "autotune needs a cell");
   double* rho_tmp = dalloc<double>(ctx.N());
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
   auto release = [&]() {
-    if (e0) cudaEventDestroy(e0);
-    if (e1) cudaEventDestroy(e1);
+    for (cudaEvent_t e : ev)
+      if (e) cudaEventDestroy(e);
     dfree(rho_tmp);
   };
-  const bool line = pencil_ok(ctx, ctx.dws, ctx.precision == MIXED);
-  double best = 1e30;
-  bool pick = ctx.fast_fft;
   try {
-    QBX_CUDA(cudaEventCreate(&e0));
-    QBX_CUDA(cudaEventCreate(&e1));
-    for (int f = line ? 1 : 0; f >= 0; f--) {
-      if (line) ctx.fast_fft = f == 1;
-      double t = 0.0;
-      for (int rep = 0; rep < 2; rep++) {   // the first pass warms up
-        QBX_CUDA(cudaEventRecord(e0, ctx.stream));
-        launch_vpsi(ctx, ctx.d_c, ctx.d_vr, ctx.d_ctmp);
-        launch_density(ctx, ctx.d_c, rho_tmp);
-        QBX_CUDA(cudaEventRecord(e1, ctx.stream));
-        QBX_CUDA(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        QBX_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        t = ms;
-      }
-      if (log) log->push_back({f ? "line passes" : "runtime-radix kernels", t});
-      if (t < best) { best = t; pick = ctx.fast_fft; }
+    for (cudaEvent_t& e : ev) QBX_CUDA(cudaEventCreate(&e));
+    float ms[2] = {0.f, 0.f};
+    for (int rep = 0; rep < 2; rep++) {   // the first pass warms up
+      QBX_CUDA(cudaEventRecord(ev[0], ctx.stream));
+      launch_vpsi(ctx, ctx.d_c, ctx.d_vr, ctx.d_ctmp);
+      QBX_CUDA(cudaEventRecord(ev[1], ctx.stream));
+      launch_density(ctx, ctx.d_c, rho_tmp);
+      QBX_CUDA(cudaEventRecord(ev[2], ctx.stream));
+      QBX_CUDA(cudaEventSynchronize(ev[2]));
+      for (int i = 0; i < 2; i++) QBX_CUDA(cudaEventElapsedTime(&ms[i], ev[i], ev[i + 1]));
+    }
+    if (log) {
+      log->push_back({"H psi", ms[0]});
+      log->push_back({"density", ms[1]});
     }
   } catch (...) {
     release();
     throw;
   }
-  ctx.fast_fft = pick;
   release();
-  return line && pick ? "line passes" : "runtime-radix kernels";
+  return pencil_ok(ctx, ctx.dws, ctx.precision == MIXED) ? "line passes" : "runtime-radix kernels";
 }
 
 }  // namespace qbx

@@ -65,9 +65,14 @@ __host__ __device__ constexpr Fac fac(int n) {
 // (the factors are template constants: evaluated in the kernels they cost
 // ten times the transform)
 template <int N> struct Keep {
-  static constexpr int r2 = fac(N).r2, pw = prune_width(N);
-  __host__ __device__ static constexpr bool q(int i) {
-    return i * r2 <= pw || i * r2 + r2 - 1 >= N - pw;
+  static constexpr int r1 = fac(N).r1, r2 = fac(N).r2, pw = prune_width(N);
+  template <bool ALL = false> __host__ __device__ static constexpr bool q(int i) {
+    return ALL || i * r2 <= pw || i * r2 + r2 - 1 >= N - pw;
+  }
+  template <bool ALL> static constexpr unsigned mask() {
+    unsigned m = 0;
+    for (int i = 0; i < r1; ++i) m |= (q<ALL>(i) ? 1u : 0u) << i;
+    return m;
   }
 };
 
@@ -93,7 +98,7 @@ template <typename T, int N, int KIND> __host__ __device__ constexpr int min_cta
   return b < 1 ? 1 : b > 8 ? 8 : b;
 }
 
-enum Op { ZB, ZF, ZBK, ZFK, YB, YF, XD, XV };
+enum Op { ZB, ZF, ZBK, ZFK, YB, YF, XD, XV, GZB, GZF, GYB, GYF, GXR, GXG };
 
 struct Args {
   DeviceSticks g;
@@ -115,6 +120,14 @@ struct Args {
   double wunit = 1;              // the sums take the weights in this unit ...
   double wout = 1;               // ... and are added to rho times this, in FP64
   bool rho_set = false;          // store the density instead of adding (chunks == 1)
+  // real fields on a whole grid (the density basis, G* passes, one slot)
+  const double2* cb = nullptr;   // second coefficient array, or null
+  double2* hcb = nullptr;
+  double* f0 = nullptr;          // the real and imaginary fields; f1 may be null
+  double* f1 = nullptr;
+  const double* fadd = nullptr;  // GXR: f0 = Re + fadd; GXG: f0, f1 times fmul
+  const double* fmul = nullptr;
+  bool chain = false;            // GXR: f1 = Im + the new f0
   cudaStream_t stream = nullptr;
 };
 
@@ -128,10 +141,11 @@ __device__ __forceinline__ void load_tw(C* tw, const double2* src) {
 
 // first half of a transform: R1-point DFT of item j and its twiddles, into
 // shared memory at [k][j] (strides sk, sj)
-template <int N, int DIR, typename C>
+template <int N, int DIR, bool ALL = false, typename C>
 __device__ __forceinline__ void first_half(C (&v)[fac(N).r1], int j, const C* tw, C* s, int sk) {
   constexpr int R1 = fac(N).r1;
-  lane::dft_reg<R1, DIR>(v);
+  constexpr unsigned MASK = Keep<N>::template mask<ALL>();
+  lane::dft_reg_in<R1, DIR, MASK>(v);
   s[0] = v[0];
 #pragma unroll
   for (int k = 1; k < R1; ++k) {
@@ -163,8 +177,9 @@ template <int N> struct ZS {
 
 // Coefficients to sticks.  One CTA takes kLines sticks of a slot; K: one
 // complex band per slot and one stick per rod, else two real bands and the
-// +G and -G sticks of each rod (stick 0 holds both halves of rod 0).
-template <typename T, int N, bool K>
+// +G and -G sticks of each rod (stick 0 holds both halves of rod 0).  G: one
+// or two real fields on the density sphere, which fills the whole line.
+template <typename T, int N, bool K, bool G = false>
 __global__ void __launch_bounds__((lines<T, N>()) * fac(N).r1, (min_ctas<T, N, KZ>()))
 zb(Args a) {
   using C = typename CT<T>::c;
@@ -177,7 +192,7 @@ zb(Args a) {
   load_tw<C, N>(tw, a.tw[2]);
   const int b1 = K ? a.first + slot : 2 * (a.first + slot);
   const double2* c1 = a.c + (size_t)b1 * a.ngw;
-  const double2* c2 = (!K && b1 + 1 < a.nst) ? c1 + a.ngw : nullptr;
+  const double2* c2 = G ? a.cb : (!K && b1 + 1 < a.nst) ? c1 + a.ngw : nullptr;
   __syncthreads();
   {
     const int j = threadIdx.x % R2, line = threadIdx.x / R2, s = s0 + line;
@@ -189,7 +204,7 @@ zb(Args a) {
 #pragma unroll
       for (int q = 0; q < R1; ++q) {
         v[q] = cmk<C>(0, 0);
-        if (Keep<N>::q(q)) {
+        if (Keep<N>::template q<G>(q)) {
           const int z = j + q * R2;
           const int lz = z < (N + 1) / 2 ? z : z - N;
           const bool minus = mstick || (!K && s == 0 && lz <= 0);
@@ -206,7 +221,7 @@ zb(Args a) {
           }
         }
       }
-      first_half<N, +1>(v, j, tw, sm + line * ZS<N>::LINE + j, ZS<N>::PJ);
+      first_half<N, +1, G>(v, j, tw, sm + line * ZS<N>::LINE + j, ZS<N>::PJ);
     }
   }
   __syncthreads();
@@ -224,9 +239,9 @@ zb(Args a) {
 }
 
 // Sticks to coefficients: hc = 1/2 g2 c + Z(G) scale, the two bands of a
-// slot unpacked at Gamma.  One CTA takes the sticks of kLines/2 rods (K:
+// slot unpacked at Gamma (G: no kinetic term).  One CTA takes the sticks of kLines/2 rods (K:
 // kLines rods).
-template <typename T, int N, bool K>
+template <typename T, int N, bool K, bool G = false>
 __global__ void __launch_bounds__((lines<T, N>()) * fac(N).r1, (min_ctas<T, N, KZ>()))
 zf(Args a) {
   using C = typename CT<T>::c;
@@ -266,7 +281,7 @@ zf(Args a) {
       C* row = sm + line * ZS<N>::LINE + j;
 #pragma unroll
       for (int q = 0; q < R1; ++q)
-        if (Keep<N>::q(q)) row[q * R2] = v[q];
+        if (Keep<N>::template q<G>(q)) row[q * R2] = v[q];
     }
   }
   __syncthreads();
@@ -279,9 +294,9 @@ zf(Args a) {
     while (r + 1 < r1 && g.rod_first[r + 1] <= ig) ++r;
     const int l = g.rod_lmin[r] + (ig - g.rod_first[r]);
     const int zp = l < 0 ? l + N : l;
-    const double kin = 0.5 * a.g2[ig];
+    const double kin = G ? 0.0 : 0.5 * a.g2[ig];
     const size_t i1 = (size_t)b1 * a.ngw + ig;
-    const double2 x = a.c[i1];
+    const double2 x = G ? make_double2(0.0, 0.0) : a.c[i1];
     if (K) {
       const C p = sm[(r - r0) * ZS<N>::LINE + zp];
       a.hc[i1] = make_double2(kin * x.x + p.x * a.scale, kin * x.y + p.y * a.scale);
@@ -295,7 +310,10 @@ zf(Args a) {
       const double px = P.x, py = P.y, mx = M.x, my = M.y;
       a.hc[i1] = make_double2(kin * x.x + 0.5 * (px + mx) * a.scale,
                               kin * x.y + 0.5 * (py - my) * a.scale);
-      if (two) {
+      if (G) {
+        if (a.hcb)
+          a.hcb[ig] = make_double2(0.5 * (py + my) * a.scale, 0.5 * (mx - px) * a.scale);
+      } else if (two) {
         const size_t i2 = i1 + a.ngw;
         const double2 y = a.c[i2];
         a.hc[i2] = make_double2(kin * y.x + 0.5 * (py + my) * a.scale,
@@ -307,7 +325,7 @@ zf(Args a) {
 
 // -------------------------------------------------------------- y columns
 // Lines (column, z) flattened; the sticks of a column through the column map.
-template <typename T, int N>
+template <typename T, int N, bool G = false>
 __global__ void __launch_bounds__((lines<T, N>()) * fac(N).r1, (min_ctas<T, N, KXY>()))
 yb(Args a) {
   using C = typename CT<T>::c;
@@ -324,7 +342,7 @@ yb(Args a) {
   if (item < R2 && on) {
 #pragma unroll
     for (int q = 0; q < R1; ++q)
-      if (Keep<N>::q(q)) {
+      if (Keep<N>::template q<G>(q)) {
         const int s = g.colmap[col * N + item + q * R2];
         off[q] = s < 0 ? -1 : s * g.n2 + z;
       }
@@ -339,7 +357,7 @@ yb(Args a) {
 #pragma unroll
     for (int q = 0; q < R1; ++q) {
       v[q] = cmk<C>(0, 0);
-      if (Keep<N>::q(q) && off[q] >= 0) v[q] = in[off[q]];
+      if (Keep<N>::template q<G>(q) && off[q] >= 0) v[q] = in[off[q]];
     }
   };
   int slot = blockIdx.y * per;
@@ -347,7 +365,7 @@ yb(Args a) {
   for (; slot < e; ++slot) {
     __syncthreads();
     if (load) {
-      first_half<N, +1>(v, item, tw, sm + item * kLines + lane, R2 * kLines);
+      first_half<N, +1, G>(v, item, tw, sm + item * kLines + lane, R2 * kLines);
       if (slot + 1 < e) fetch(slot + 1);   // in flight over the second half
     }
     __syncthreads();
@@ -363,7 +381,7 @@ yb(Args a) {
   }
 }
 
-template <typename T, int N>
+template <typename T, int N, bool G = false>
 __global__ void __launch_bounds__((lines<T, N>()) * fac(N).r1, (min_ctas<T, N, KXY>()))
 yf(Args a) {
   using C = typename CT<T>::c;
@@ -380,7 +398,7 @@ yf(Args a) {
   if (item < R2 && on) {
 #pragma unroll
     for (int q = 0; q < R1; ++q)
-      if (Keep<N>::q(q)) {
+      if (Keep<N>::template q<G>(q)) {
         const int s = g.colmap[col * N + item + q * R2];
         off[q] = s < 0 ? -1 : s * g.n2 + z;
       }
@@ -411,7 +429,7 @@ yf(Args a) {
       C* out = (C*)a.sticks + slot * zs;
 #pragma unroll
       for (int q = 0; q < R1; ++q)
-        if (Keep<N>::q(q) && off[q] >= 0) out[off[q]] = v[q];
+        if (Keep<N>::template q<G>(q) && off[q] >= 0) out[off[q]] = v[q];
     }
   }
 }
@@ -558,6 +576,88 @@ xv(Args a) {
   }
 }
 
+// One complex transform of real fields on the whole grid: the tile to f0 (and
+// f1), or back from them.  The pointwise work next to it rides along: f0 takes
+// fadd (v_xc += ...), f1 the new f0 (V = V_local + v_xc), the fields to be
+// transformed are multiplied by fmul.
+template <int N>
+__global__ void __launch_bounds__((lines<double, N>()) * fac(N).r1, (min_ctas<double, N, KXY>()))
+xr(Args a) {
+  using C = double2;
+  constexpr int R1 = fac(N).r1, R2 = fac(N).r2, kLines = lines<double, N>();
+  __shared__ C tw[N];
+  __shared__ C sm[N * kLines];
+  const DeviceSticks& g = a.g;
+  const int lane = threadIdx.x % kLines, item = threadIdx.x / kLines;
+  const int line = blockIdx.x * kLines + lane;
+  const int nl = g.n1 * g.n2;
+  const bool on = line < nl;
+  load_tw<C, N>(tw, a.tw[0]);
+  C v[R1];
+  if (item < R2 && on) {
+    const C* in = (const C*)a.tile + line;
+#pragma unroll
+    for (int q = 0; q < R1; ++q) {
+      const int col = g.xcol[item + q * R2];
+      v[q] = col >= 0 ? in[(size_t)col * nl] : make_double2(0.0, 0.0);
+    }
+  }
+  __syncthreads();
+  if (item < R2 && on) first_half<N, +1, true>(v, item, tw, sm + item * kLines + lane, R2 * kLines);
+  __syncthreads();
+  if (!on) return;
+  C u[R2];
+#pragma unroll
+  for (int j = 0; j < R2; ++j) u[j] = sm[(item * R2 + j) * kLines + lane];
+  lane::dft_reg<R2, +1>(u);
+#pragma unroll
+  for (int m = 0; m < R2; ++m) {
+    const size_t p = (size_t)(item + m * R1) * nl + line;
+    const double f = a.fadd ? u[m].x + a.fadd[p] : u[m].x;
+    a.f0[p] = f;
+    if (a.f1) a.f1[p] = a.chain ? u[m].y + f : u[m].y;
+  }
+}
+
+template <int N>
+__global__ void __launch_bounds__((lines<double, N>()) * fac(N).r1, (min_ctas<double, N, KXY>()))
+xg(Args a) {
+  using C = double2;
+  constexpr int R1 = fac(N).r1, R2 = fac(N).r2, kLines = lines<double, N>();
+  __shared__ C tw[N];
+  __shared__ C sm[N * kLines];
+  const DeviceSticks& g = a.g;
+  const int lane = threadIdx.x % kLines, item = threadIdx.x / kLines;
+  const int line = blockIdx.x * kLines + lane;
+  const int nl = g.n1 * g.n2;
+  const bool on = line < nl;
+  load_tw<C, N>(tw, a.tw[0]);
+  C u[R2];
+  if (on) {
+#pragma unroll
+    for (int m = 0; m < R2; ++m) {
+      const size_t p = (size_t)(item + m * R1) * nl + line;
+      const double w = a.fmul ? a.fmul[p] : 1.0;
+      u[m] = make_double2(a.f0[p] * w, a.f1 ? a.f1[p] * w : 0.0);
+    }
+  }
+  __syncthreads();
+  if (on) first_half_rev<N, -1>(u, item, tw, sm + item * R2 * kLines + lane, kLines);
+  __syncthreads();
+  if (item < R2 && on) {
+    C v[R1];
+#pragma unroll
+    for (int k = 0; k < R1; ++k) v[k] = sm[(k * R2 + item) * kLines + lane];
+    lane::dft_reg<R1, -1>(v);
+    C* out = (C*)a.tile + line;
+#pragma unroll
+    for (int q = 0; q < R1; ++q) {
+      const int col = g.xcol[item + q * R2];
+      if (col >= 0) out[(size_t)col * nl] = v[q];
+    }
+  }
+}
+
 // -------------------------------------------------- lines of a whole grid
 // In place, FP64, every line along one axis of an x-fastest grid.  Along y and
 // z the neighbouring lines are neighbours in memory (inner of them, then the
@@ -583,7 +683,7 @@ gs(double2* __restrict__ grid, const double2* __restrict__ tw_g, int inner, int 
   }
   __syncthreads();
   if (item < R2 && on)
-    first_half<N, DIR>(v, item, tw, sm + item * kLines + lane, R2 * kLines);
+    first_half<N, DIR, true>(v, item, tw, sm + item * kLines + lane, R2 * kLines);
   __syncthreads();
   if (on) {
     C u[R2];
@@ -613,7 +713,7 @@ gc(double2* __restrict__ grid, const double2* __restrict__ tw_g, int nlines) {
     for (int q = 0; q < R1; ++q) v[q] = in[q * R2];
   }
   __syncthreads();
-  if (on) first_half<N, DIR>(v, j, tw, sm + lj * ZS<N>::LINE + j, ZS<N>::PJ);
+  if (on) first_half<N, DIR, true>(v, j, tw, sm + lj * ZS<N>::LINE + j, ZS<N>::PJ);
   __syncthreads();
   const int k = threadIdx.x % R1, line = threadIdx.x / R1;
   if (line < kLines && l0 + line < nlines) {
@@ -662,8 +762,15 @@ void run(Context& ctx, const Args& a) {
     case XV: xv<T, N><<<gx, th, 0, st>>>(a); break;
     default:
       if constexpr (sizeof(T) == 8) {
-        if (a.op == ZBK) zb<T, N, true><<<dim3(cdiv(g.nvec, kLines), a.nslots), th, 0, st>>>(a);
-        else zf<T, N, true><<<dim3(cdiv(g.nrods, kLines), a.nslots), th, 0, st>>>(a);
+        const dim3 gzb(cdiv(g.nvec, kLines), a.nslots);
+        if (a.op == ZBK) zb<T, N, true><<<gzb, th, 0, st>>>(a);
+        else if (a.op == ZFK) zf<T, N, true><<<dim3(cdiv(g.nrods, kLines), a.nslots), th, 0, st>>>(a);
+        else if (a.op == GZB) zb<T, N, false, true><<<gzb, th, 0, st>>>(a);
+        else if (a.op == GZF) zf<T, N, false, true><<<cdiv(g.nrods, kLines / 2), th, 0, st>>>(a);
+        else if (a.op == GYB) yb<T, N, true><<<gy, th, 0, st>>>(a);
+        else if (a.op == GYF) yf<T, N, true><<<gy, th, 0, st>>>(a);
+        else if (a.op == GXR) xr<N><<<gx, th, 0, st>>>(a);
+        else xg<N><<<gx, th, 0, st>>>(a);
       }
   }
   QBX_LAUNCHED(ctx);

@@ -165,11 +165,6 @@ __global__ void k_mul(const double* __restrict__ a, const double* __restrict__ b
     out[i] = a[i] * b[i];
 }
 
-__global__ void k_axpy(double* __restrict__ y, const double* __restrict__ x, size_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x)
-    y[i] += x[i];
-}
 
 // sum_i x_i y_i
 struct DotF {
@@ -195,7 +190,6 @@ void launch_xc(Context& ctx) {
     k_lda<<<nb, kThreads, 0, ctx.stream>>>(ctx.d_rhor, N, ctx.d_vxc, ctx.d_exc);
     QBX_LAUNCHED(ctx);
     launch_sum(ctx, ctx.d_exc, N, SLOT_EXC);
-    reduce<1>(ctx, DotF{ctx.d_rhor, ctx.d_vxc}, N, SLOT_EXC + 2);   // for dxc
     return;
   }
   // PBE: grad rho as the backward transforms of i G_j rho(G)/Omega, two real
@@ -215,18 +209,14 @@ void launch_xc(Context& ctx) {
   QBX_LAUNCHED(ctx);
   // sum e_xc and sum rho v1 (the latter for the XC stress)
   reduce<2>(ctx, SumRhoV1F{ctx.d_exc, ctx.d_rhor, ctx.d_vxc}, N, SLOT_EXC);
-  // vxc += backward(sum_j i G_j forward(grad_j vxc2)): the forward transforms
-  // two real fields to a complex one, the sum in G space before one backward
+  // the divergence term sum_j i G_j forward(grad_j vxc2) in G space, two real
+  // fields to a complex transform; launch_vhxc_rspace takes it back to r
   vb_forward_real_pair(ctx, ctx.d_grad, ctx.d_grad + N, ctx.d_vx2, xg[0], xg[1]);
   vb_forward_real_pair(ctx, ctx.d_grad + 2 * N, nullptr, ctx.d_vx2, xg[2], nullptr);
   k_sum_igx3<<<blocks_for(ngv), kThreads, 0, ctx.stream>>>(
       (const double2*)xg[0], (const double2*)xg[1], (const double2*)xg[2], ctx.d_gx_v, ngv,
       (double2*)ctx.d_vtmp_g);
   QBX_LAUNCHED(ctx);
-  vb_backward(ctx, ctx.d_vtmp_g, ctx.d_exc);
-  k_axpy<<<nb, kThreads, 0, ctx.stream>>>(ctx.d_vxc, ctx.d_exc, N);
-  QBX_LAUNCHED(ctx);
-  reduce<1>(ctx, DotF{ctx.d_rhor, ctx.d_vxc}, N, SLOT_EXC + 2);   // for dxc
 }
 
 // ---------------------------------------------------- Hartree and local
@@ -268,11 +258,18 @@ void launch_vhxc_gspace(Context& ctx) {
             (size_t)ngv, SLOT_EPS_EH);
   k_vlocal_g<<<blocks_for(ngv), kThreads, 0, ctx.stream>>>(
       (const double2*)ctx.d_rhog, (const double2*)ctx.d_vion, (const double2*)ctx.d_rhops,
-      ctx.d_g2i_v, ngv, 1.0 / om, (double2*)ctx.d_vtmp_g, (double2*)ctx.d_vtmp_g2);
+      ctx.d_g2i_v, ngv, 1.0 / om, (double2*)ctx.d_xc_g, (double2*)ctx.d_vtmp_g2);
   QBX_LAUNCHED(ctx);
-  vb_backward(ctx, ctx.d_vtmp_g, ctx.d_vr);
-  k_axpy<<<blocks_for(ctx.N()), kThreads, 0, ctx.stream>>>(ctx.d_vr, ctx.d_vxc, ctx.N());
-  QBX_LAUNCHED(ctx);
+}
+
+// Back to r: v_xc takes the GGA's divergence term and V(r) = V_local + v_xc, the
+// two fields in one complex transform; then sum rho v_xc (for dxc).
+void launch_vhxc_rspace(Context& ctx) {
+  if (ctx.xc == "LDA")
+    vb_backward_add(ctx, ctx.d_xc_g, nullptr, ctx.d_vxc, ctx.d_vr, nullptr);
+  else
+    vb_backward_add(ctx, ctx.d_vtmp_g, ctx.d_xc_g, ctx.d_vxc, ctx.d_vxc, ctx.d_vr);
+  reduce<1>(ctx, DotF{ctx.d_rhor, ctx.d_vxc}, ctx.N(), SLOT_EXC + 2);
 }
 
 // ------------------------------------------------- wavefunction sums

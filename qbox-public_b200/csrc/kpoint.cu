@@ -386,7 +386,10 @@ void set_kpoints(Context& ctx, int nk, const double* k, const double* w) {
     }
   }
   free_kpoints(ctx);
-  if (nk == 0) return;
+  if (nk == 0) {
+    kpoints_grid_order(ctx);
+    return;
+  }
   const int n = ctx.nst;
   ctx.kpts.resize(nk);
   for (int i = 0; i < nk; i++) {
@@ -413,6 +416,7 @@ void set_kpoints(Context& ctx, int nk, const double* k, const double* w) {
   }
   ctx.d_znn = dalloc<double>(6 * 2 * (size_t)n * n);
   ensure_zwork(ctx);
+  kpoints_grid_order(ctx);
 }
 
 // SlaterDet::gram, complex branch (src/SlaterDet.cpp:524-533): C <- C L^-H

@@ -460,6 +460,7 @@ struct Context {
   size_t zfast_bytes = 0;
   bool fast_fft = true;         // the line-pass FFTs (fft_pencil.cuh) where they take the grid
   float* a32 = nullptr;         // TF32 hi/lo split of the projectors
+  bool grid_zfast = false;      // the real-space grids are kept z fastest (fft.cu)
   float* a32lo = nullptr;
   float* s32 = nullptr;         // TF32 hi/lo split of a small matrix
   float* s32lo = nullptr;
@@ -594,6 +595,15 @@ void vb_forward_real_pair(Context& ctx, const double* f0, const double* f1, cons
                           double* c0, double* c1);
 // wavefunction-basis single transforms through the full-grid path (tests)
 void wb_backward_pair(Context& ctx, const double* c1, const double* c2, double* grid_out);
+// out0 = add + back(a); with b also out1 = out0 + back(b) (d_exc is scratch)
+void vb_backward_add(Context& ctx, const double* a, const double* b, const double* add,
+                     double* out0, double* out1);
+// whether the grids can be kept z fastest, and their conversion from and to
+// the callers' x-fastest order (device arrays)
+bool grid_zfast_possible(const Context& ctx);
+void kpoints_grid_order(Context& ctx);   // after the set of k points changed
+void grid_to_caller(Context& ctx, const double* f, double* out);
+void grid_from_caller(Context& ctx, const double* f, double* out);
 
 // staged-FFT launch configuration by timing on the context's own data
 std::string autotune_fft(Context& ctx, std::vector<std::pair<std::string, double>>* log);
@@ -604,7 +614,8 @@ double* density_weights(Context& ctx);
 // pointwise kernels (kernels.cu)
 void launch_sum(Context& ctx, const double* x, size_t n, int slot);   // slot = sum x
 void launch_xc(Context& ctx);                  // fills d_vxc; SLOT_EXC
-void launch_vhxc_gspace(Context& ctx);         // SLOT_EPS_EH, vlocal_g
+void launch_vhxc_gspace(Context& ctx);         // SLOT_EPS_EH, V_local(G)
+void launch_vhxc_rspace(Context& ctx);         // v_xc complete, V(r), SLOT_EXC + 2
 void launch_setup_atoms(Context& ctx);         // sfac, vion, rhops, anl
 void launch_ekin(Context& ctx);                // SLOT_EKIN
 void launch_eigsum(Context& ctx);              // SLOT_EIG

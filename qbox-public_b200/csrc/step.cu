@@ -590,6 +590,7 @@ static void nonlocal(Context& ctx, bool hpsi) {
       QBX_BLAS(cublasDgemm(ctx.blas, CUBLAS_OP_T, CUBLAS_OP_N, np, n, K, &two, ctx.d_anl, K,
                            ctx.d_c, K, &zero, ctx.d_fnl, np));
   }
+  launch_vhxc_rspace(ctx);
   launch_rank1_fix(ctx, ctx.d_fnl, np, ctx.d_anl, K, ctx.d_c, K, np, n, -1.0, false);
   launch_enl(ctx);
   if (hpsi) {
