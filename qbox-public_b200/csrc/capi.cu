@@ -1628,7 +1628,7 @@ int qbx_split_gemm_tn(qbx_context* h, int m, int n, int k, const double* a, cons
         c.d_acc32 = acc;
         c.acc32_elems = (size_t)m * n;
         c.gemm_backend = backend;
-        QBX_REQUIRE(backend == 0 || tc_gemm_supported(c, true, false, m, n, k), 54,
+        QBX_REQUIRE(backend == 0 || tc_gemm_whole_tiles(true, false, m, n, k), 54,
                     "shape not supported by the tcgen05 GEMM");
         split_gemm(c, true, false, m, n, k, 1.0, ah, al, ldp, bh, bl, ldp, 0.0, dd);
       }

@@ -1205,7 +1205,7 @@ void compute_stress_nl(Context& ctx) {
     const int K = 2 * ngw;
     if (!ctx.d_astress) ctx.d_astress = dalloc<double>((size_t)K * np);
     const bool mx = ctx.precision == MIXED && ctx.gemm_backend == 1 &&
-                    tc_gemm_supported(ctx, true, false, np, nst, K);
+                    tc_gemm_whole_tiles(true, false, np, nst, K);
     if (mx && !ctx.sa_hi) {
       QBX_CUDA(cudaMalloc(&ctx.sa_hi, (size_t)ctx.ldp * np * 2));
       QBX_CUDA(cudaMalloc(&ctx.sa_lo, (size_t)ctx.ldp * np * 2));

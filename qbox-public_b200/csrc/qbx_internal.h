@@ -759,7 +759,9 @@ void overlap_diag_f64(Context& ctx, const double* c, int K, int n, double* S);
 void split_gemm(Context& ctx, bool ta, bool tb, int m, int n, int k, double alpha,
                 const void* ahi, const void* alo, int lda, const void* bhi, const void* blo,
                 int ldb, double beta, double* C, bool lower = false);
-bool tc_gemm_supported(const Context& ctx, bool ta, bool tb, int m, int n, int k);
+bool tc_gemm_supported(bool ta, bool tb, int m, int n, int k);
+// of these, the products of whole 128 x 128 tiles
+bool tc_gemm_whole_tiles(bool ta, bool tb, int m, int n, int k);
 void tc_split_gemm(Context& ctx, bool ta, bool tb, int m, int n, int k, double alpha,
                    const void* ahi, const void* alo, int lda, const void* bhi, const void* blo,
                    int ldb, double beta, double* C, bool lower = false);
