@@ -83,7 +83,7 @@ void free_cell(Context& c) {
   double** bufs[] = {&c.d_gx_w, &c.d_g2_w, &c.d_gx_v, &c.d_g2i_v, &c.d_c, &c.d_hc, &c.d_c_last,
                      &c.d_dc_last, &c.d_ctmp, &c.d_occ, &c.d_rhor, &c.d_vr, &c.d_vxc,
                      &c.d_exc, &c.d_vx2, &c.d_grad, &c.d_rhog, &c.d_vion, &c.d_rhops,
-                     &c.d_vtmp_g, &c.d_vtmp_g2, &c.d_xc_g, &c.d_nn, &c.d_nn2, &c.d_nn3, &c.d_nn4, &c.d_nn5,
+                     &c.d_vtmp_g, &c.d_vtmp_g2, &c.d_xc_g, &c.d_nn, &c.d_nn2, &c.d_nn3, &c.d_nn4, &c.d_nn5, &c.d_small,
                      &c.d_solver_work, &c.d_red, &c.d_scalars, &c.d_prec, &c.d_jd_h,
                      &c.d_jd_w, &c.d_jd_work, &c.d_wfv, &c.d_xsd, &c.d_xgrid};
   for (double** b : bufs) dfree(*b);
@@ -397,6 +397,7 @@ int qbx_create(qbx_context** out, int device, int precision) {
   if (const char* e = std::getenv("QBX_TC_PAIR")) h->c.tc_pair = std::max(0, std::min(2, std::atoi(e)));
   if (const char* e = std::getenv("QBX_TC_PAIR_EPW")) h->c.tc_pair_epw = std::atoi(e) == 8 ? 8 : 16;
   if (const char* e = std::getenv("QBX_TC_TF32_MN")) h->c.tc_tf32_mn = std::atoi(e) != 0 ? 1 : 0;
+  if (const char* e = std::getenv("QBX_ORTHO_SMALL")) h->c.ortho_small = std::atoi(e) != 0 ? 1 : 0;
   if (const char* e = std::getenv("QBX_STEP_FUSE")) h->c.step_fuse = std::atoi(e) != 0 ? 1 : 0;
   if (const char* e = std::getenv("QBX_TC_CORR_MUL")) h->c.tc_corr_mul = std::max(0, std::min(64, std::atoi(e)));
   if (const char* e = std::getenv("QBX_TALL_KIND_HC")) h->c.tall_kind_hc = std::atoi(e) == 1 ? 1 : 0;
@@ -531,6 +532,7 @@ int qbx_set_cell(qbx_context* h, const double cell[9], double ecut, int nst, con
     c.d_nn3 = dalloc<double>(nn);
     c.d_nn4 = dalloc<double>(3 * nn);
     c.d_nn5 = dalloc<double>(nn);
+    c.d_small = dalloc<double>(ortho_small_elems(nst));
     c.d_ipiv = dalloc<int>(nst);
     c.d_info = dalloc<int>(1);
     int lw1 = 0, lw2 = 0;
@@ -561,9 +563,9 @@ int qbx_set_cell(qbx_context* h, const double cell[9], double ecut, int nst, con
       if (const char* e = std::getenv("QBX_FAST_FFT")) c.fast_fft = std::atoi(e) != 0;
       if (const char* e = std::getenv("QBX_PSIR")) c.wtile_mode = std::atoi(e) != 0 ? 1 : 0;
     }
+    c.grid_zfast = grid_zfast_possible(c);
     c.species.clear();
     c.tau.clear();
-    c.grid_zfast = grid_zfast_possible(c);
     QBX_CUDA(cudaDeviceSynchronize());   // memsets above ran on the legacy stream
     c.have_cell = true;
     alloc_mixed(c);

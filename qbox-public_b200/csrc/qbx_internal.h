@@ -376,6 +376,8 @@ struct Context {
   double* d_nn3 = nullptr;
   double* d_nn4 = nullptr;
   double* d_nn5 = nullptr;      // n x n: L^-1 of ortho_align's overlap (mixed path)
+  double* d_small = nullptr;    // workspace of ortho_small.cu (up to 128 bands)
+  int ortho_small = 1;          // ortho_align's n x n algebra in one kernel where it fits
   int* d_ipiv = nullptr;
   int* d_info = nullptr;
   double* d_solver_work = nullptr;
@@ -458,9 +460,9 @@ struct Context {
   float* d_vr32 = nullptr;      // FP32 copy of V(r) for the mixed H*psi pass
   void* d_zfast = nullptr;      // stick buffer of the specialised staged FFTs
   size_t zfast_bytes = 0;
+  bool grid_zfast = false;      // the real-space grids are kept z fastest (fft.cu)
   bool fast_fft = true;         // the line-pass FFTs (fft_pencil.cuh) where they take the grid
   float* a32 = nullptr;         // TF32 hi/lo split of the projectors
-  bool grid_zfast = false;      // the real-space grids are kept z fastest (fft.cu)
   float* a32lo = nullptr;
   float* s32 = nullptr;         // TF32 hi/lo split of a small matrix
   float* s32lo = nullptr;
@@ -593,8 +595,6 @@ void vb_backward_pair(Context& ctx, const double* a, const double* b, double* ou
 // transform, with the 1/N of the forward transform
 void vb_forward_real_pair(Context& ctx, const double* f0, const double* f1, const double* w,
                           double* c0, double* c1);
-// wavefunction-basis single transforms through the full-grid path (tests)
-void wb_backward_pair(Context& ctx, const double* c1, const double* c2, double* grid_out);
 // out0 = add + back(a); with b also out1 = out0 + back(b) (d_exc is scratch)
 void vb_backward_add(Context& ctx, const double* a, const double* b, const double* add,
                      double* out0, double* out1);
@@ -604,6 +604,8 @@ bool grid_zfast_possible(const Context& ctx);
 void kpoints_grid_order(Context& ctx);   // after the set of k points changed
 void grid_to_caller(Context& ctx, const double* f, double* out);
 void grid_from_caller(Context& ctx, const double* f, double* out);
+// wavefunction-basis single transforms through the full-grid path (tests)
+void wb_backward_pair(Context& ctx, const double* c1, const double* c2, double* grid_out);
 
 // staged-FFT launch configuration by timing on the context's own data
 std::string autotune_fft(Context& ctx, std::vector<std::pair<std::string, double>>* log);
@@ -711,6 +713,13 @@ void polar_factor(Context& ctx, double* x, double tol, int maxiter);
 // of two (work: n * n / 4 doubles), else a triangular solve of I
 bool lower_inverse_blocked(int n);
 void lower_inverse(Context& ctx, const double* L, int n, double* Li, double* work);
+// The n x n algebra of ortho_align and polar in one kernel (ortho_small.cu), up
+// to 128 bands: X = L^-T polar(L^-1 B) with S = L L^T (lower triangle), I - X
+// into IX unless null, the factorisation's info code into status word `info`
+bool ortho_small_ok(const Context& ctx);
+size_t ortho_small_elems(int n);   // of Context::d_small; 0: too many bands
+void ortho_small(Context& ctx, const double* S, const double* B, double* X, double* IX, int info);
+void polar_small(Context& ctx, double* x, double tol, int maxiter);
 int polar_entry(Context& ctx, double* x, double tol, int maxiter, bool graph);
 // one electronic step (captured graph or eager), energies/fion as qbx_scf_step
 void scf_step_any(Context& c, bool want_f, bool want_s, double* energies, double* fion);

@@ -20,14 +20,12 @@ namespace qbx {
 
 static bool mixed(const Context& ctx) { return ctx.precision == MIXED; }
 
-// S = 2 C^T C - c0 c0^T, lower triangle, then S = L L^T in place.  In the
+// S = 2 C^T C - c0 c0^T, lower triangle; overlap_cholesky: then S = L L^T in place.  In the
 // mixed path the product uses the BF16 split of c in slot `split` and the
 // diagonal is recomputed exactly in FP64.  The factorisation's info code
 // goes to the status word `status` (checked when the step's scalars are
 // read back: a matrix that is not positive definite is an error there).
-static void overlap_cholesky(Context& ctx, const double* c, double* S, int status, int split,
-                             bool diag_from_split = false) {
-  ProfScope ps(ctx, "overlap_cholesky");
+static void overlap(Context& ctx, const double* c, double* S, int split, bool diag_from_split) {
   const int n = ctx.nst, K = 2 * ctx.wb.ng;
   const double two = 2.0, zero = 0.0;
   if (split >= 0) {
@@ -42,8 +40,13 @@ static void overlap_cholesky(Context& ctx, const double* c, double* S, int statu
                          S, n));
     launch_rank1_fix(ctx, S, n, c, K, c, K, n, n, -1.0, true);
   }
-  QBX_SOLVER(cusolverDnDpotrf(ctx.solver, CUBLAS_FILL_MODE_LOWER, n, S, n, ctx.d_solver_work,
-                              ctx.solver_lwork, ctx.d_status + status));
+}
+static void overlap_cholesky(Context& ctx, const double* c, double* S, int status, int split,
+                             bool diag_from_split = false) {
+  ProfScope ps(ctx, "overlap_cholesky");
+  overlap(ctx, c, S, split, diag_from_split);
+  QBX_SOLVER(cusolverDnDpotrf(ctx.solver, CUBLAS_FILL_MODE_LOWER, ctx.nst, S, ctx.nst,
+                              ctx.d_solver_work, ctx.solver_lwork, ctx.d_status + status));
 }
 
 static void rotate(Context& ctx, double* x, const double* M);
@@ -287,6 +290,7 @@ void capture_body(Context& ctx, cudaGraph_t body, cudaStream_t s, const std::fun
 
 static void polar(Context& ctx, double* x, double tol, int maxiter) {
   ProfScope ps(ctx, "polar");
+  if (ortho_small_ok(ctx)) return polar_small(ctx, x, tol, maxiter);
   const int n = ctx.nst;
   double* q = ctx.d_nn3;
   double* t = ctx.d_nn4;
@@ -348,6 +352,11 @@ void polar_factor(Context& ctx, double* x, double tol, int maxiter) { polar(ctx,
 int polar_entry(Context& ctx, double* x, double tol, int maxiter, bool graph) {
   if (!graph) {
     polar(ctx, x, tol, maxiter);
+    if (ortho_small_ok(ctx)) {
+      QBX_CUDA(cudaMemcpyAsync(&ctx.polar_iters, ctx.d_status + ST_POLAR_ITERS, sizeof(int),
+                               cudaMemcpyDeviceToHost, ctx.stream));
+      QBX_CUDA(cudaStreamSynchronize(ctx.stream));
+    }
     return ctx.polar_iters;
   }
   const bool prof = ctx.prof.on;
@@ -441,7 +450,13 @@ void ortho_align(Context& ctx, bool c_split_done) {
                     (float*)ctx.ct_lo, ctx.ldp);
   else if (mx && !both)
     split_bf16_2d(ctx, ctx.d_c, K, n, K, ctx.cs_hi[1], ctx.cs_lo[1], ctx.ldp);
-  overlap_cholesky(ctx, ctx.d_c, L, ST_INFO_ORTHO, mx ? 1 : -1, both);
+  const bool small = ortho_small_ok(ctx);   // the n x n algebra in one kernel
+  if (small) {
+    ProfScope ps(ctx, "overlap_cholesky");
+    overlap(ctx, ctx.d_c, L, mx ? 1 : -1, both);
+  } else {
+    overlap_cholesky(ctx, ctx.d_c, L, ST_INFO_ORTHO, mx ? 1 : -1, both);
+  }
   // B = 2 C^T C_last - c0 c_last0^T
   {
     ProfScope ps(ctx, "gemm_overlap_last");
@@ -453,7 +468,10 @@ void ortho_align(Context& ctx, bool c_split_done) {
                            ctx.d_c_last, K, &zero, X, n));
   }
   launch_rank1_fix(ctx, X, n, ctx.d_c, K, ctx.d_c_last, K, n, n, -1.0, false);
-  if (mx) {
+  if (small) {
+    ProfScope ps(ctx, "polar");
+    ortho_small(ctx, L, X, X, mx ? ctx.d_nn3 : nullptr, ST_INFO_ORTHO);
+  } else if (mx) {
     // L^-1 once (one triangular solve of I), then two products in place of
     // the two solves with L and L^T (each solve as slow as the inverse)
     double* Li = ctx.d_nn5;
@@ -476,7 +494,7 @@ void ortho_align(Context& ctx, bool c_split_done) {
     // C <- C - C (I - X): the split-precision error only touches the
     // correction, so C stays orthonormal to the accuracy of the overlap.
     double* T = ctx.d_nn3;
-    launch_identity_axpy(ctx, T, X, n, -1.0);
+    if (!small) launch_identity_axpy(ctx, T, X, n, -1.0);
     // rotation: TF32 splits, so that C stays orthonormal to ~1e-7
     tall_update(ctx, ctx.tall_kind, ctx.d_c, T, -1.0, ctx.d_c, both ? ctx.ct_hi : nullptr,
                 both ? ctx.ct_lo : nullptr);
@@ -572,6 +590,7 @@ void update_vhxc(Context& ctx) {
   ProfScope ps(ctx, "update_vhxc");
   launch_xc(ctx);
   launch_vhxc_gspace(ctx);
+  launch_vhxc_rspace(ctx);
 }
 
 // NonLocalPotential::energy (src/NonLocalPotential.cpp:1258-1640):
@@ -590,7 +609,6 @@ static void nonlocal(Context& ctx, bool hpsi) {
       QBX_BLAS(cublasDgemm(ctx.blas, CUBLAS_OP_T, CUBLAS_OP_N, np, n, K, &two, ctx.d_anl, K,
                            ctx.d_c, K, &zero, ctx.d_fnl, np));
   }
-  launch_vhxc_rspace(ctx);
   launch_rank1_fix(ctx, ctx.d_fnl, np, ctx.d_anl, K, ctx.d_c, K, np, n, -1.0, false);
   launch_enl(ctx);
   if (hpsi) {

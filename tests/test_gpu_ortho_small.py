@@ -1,0 +1,80 @@
+"""The n x n algebra of ortho_align and polar in one kernel (up to 128 bands)
+against the library chain (QBX_ORTHO_SMALL=0): the panel remainders, one and
+eight panels, both branches of the polar iteration in both precisions, captured
+and eager, and a factorisation that fails.
+
+Both are FP64 throughout; they differ in the order of sums and in forming L^-1
+explicitly, so to some n eps times the condition of the overlap (10 here):
+1e-11.
+"""
+import os
+
+import numpy as np
+import pytest
+
+from qbx import capi, systems
+
+pytestmark = pytest.mark.gpu
+
+BANDS = [1, 7, 15, 16, 17, 40, 97, 127, 128]
+
+
+def _ctx(bands, precision, small, xc="LDA"):
+    pos = systems.diamond_supercell(10.26, 1, 0.03, 4)[:5]
+    s = systems.System("box", np.diag([11.0, 10.0, 12.5]), [systems.SI], [(0, p) for p in pos],
+                       20.0, bands, xc, 13)
+    os.environ["QBX_ORTHO_SMALL"] = small
+    try:
+        return capi.from_system(s, precision=precision)
+    finally:
+        os.environ.pop("QBX_ORTHO_SMALL")
+
+
+@pytest.mark.parametrize("precision", [capi.FP64, capi.MIXED])
+@pytest.mark.parametrize("n", BANDS)
+def test_polar(n, precision):
+    rng = np.random.default_rng(n)
+    q, _ = np.linalg.qr(rng.standard_normal((n, n)))
+    near = q @ (np.eye(n) + 0.02 / n * rng.standard_normal((n, n)))
+    far = q @ np.diag(np.linspace(0.4, 2.5, n)) @ np.linalg.qr(rng.standard_normal((n, n)))[0]
+    ctx = _ctx(n, precision, "1")
+    for x in (near, far):
+        u, _, vt = np.linalg.svd(x)
+        for graph in (False, True):
+            f, it = ctx.polar(x, 1e-6, 20, graph)
+            np.testing.assert_allclose(f, u @ vt, rtol=0, atol=1e-11)
+            assert 1 <= it <= 12
+    ctx.close()
+
+
+@pytest.mark.parametrize("precision", [capi.FP64, capi.MIXED])
+@pytest.mark.parametrize("n", BANDS)
+def test_step_matches_library_chain(n, precision):
+    out = []
+    for small in ("1", "0"):
+        ctx = _ctx(n, precision, small)
+        e = [ctx.scf_step()["etotal"] for _ in range(2)]
+        ctx.set_step_graph(True)
+        e += [ctx.scf_step()["etotal"] for _ in range(2)]
+        out.append((np.array(e), ctx.get_coeffs()))
+        ctx.close()
+    (ea, ca), (eb, cb) = out
+    np.testing.assert_allclose(ea, eb, rtol=1e-11)
+    np.testing.assert_allclose(ca, cb, rtol=0, atol=1e-10 if precision == capi.FP64 else 1e-7)
+
+
+@pytest.mark.parametrize("precision", [capi.FP64, capi.MIXED])
+def test_singular_overlap_is_an_error(precision):
+    ctx = _ctx(20, precision, "1")
+    c = ctx.get_coeffs()
+    bad = c.copy()
+    bad[7] = 0.0
+    ctx.set_coeffs(bad)
+    with pytest.raises(capi.QbxError):
+        ctx.ortho_align(c)
+    # the context goes on
+    ctx.set_coeffs(c)
+    ctx.ortho_align(c)
+    np.testing.assert_allclose(ctx.get_coeffs(), c, rtol=0,
+                               atol=1e-11 if precision == capi.FP64 else 1e-6)
+    ctx.close()
