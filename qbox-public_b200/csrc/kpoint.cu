@@ -201,10 +201,11 @@ void ensure_zwork(Context& ctx) {
 // scalars are read back (no host read inside a step)
 void overlap_cholesky_k(Context& ctx, const double* c, int ngw, int status) {
   const int n = ctx.nst;
-  const double one = 1.0, zero = 0.0;
   double* L = znn(ctx, 0);
-  QBX_BLAS(cublasZherk(ctx.blas, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_C, n, ngw, &one, zc(c), ngw,
-                       &zero, zc(L), n));
+  // the whole product: cuBLAS's herk does not split the long contraction
+  // (n = 128, 24 k rows: 0.84 ms against 0.13)
+  QBX_BLAS(cublasZgemm(ctx.blas, CUBLAS_OP_C, CUBLAS_OP_N, n, n, ngw, &kOne, zc(c), ngw, zc(c),
+                       ngw, &kZero, zc(L), n));
   QBX_SOLVER(cusolverDnZpotrf(ctx.solver, CUBLAS_FILL_MODE_LOWER, n, zc(L), n, zc(ctx.d_zwork),
                               ctx.zwork_len, ctx.d_status + status));
 }
