@@ -177,7 +177,8 @@ __device__ __forceinline__ void dft_in(C (&v)[R]) {
       const bool p = (MASK >> m) & 1, q = (MASK >> (R - m)) & 1;
       if (!p && !q) continue;
       a[m] = p && q ? cadd(v[m], v[R - m]) : p ? v[m] : v[R - m];
-      b[m] = p && q ? csub(v[m], v[R - m]) : p ? v[m] : cmk<C>(-v[R - m].x, -v[R - m].y);
+      b[m] = reg::cmuli<DIR>(p && q ? csub(v[m], v[R - m])
+                                    : p ? v[m] : cmk<C>(-v[R - m].x, -v[R - m].y));
       s0 = any ? cadd(s0, a[m]) : a[m];
       any = true;
     }
@@ -185,20 +186,16 @@ __device__ __forceinline__ void dft_in(C (&v)[R]) {
     out[0] = s0;
 #pragma unroll
     for (int k = 1; k <= H; ++k) {
-      Real rx = v0.x, ry = v0.y, ix = 0, iy = 0;
+      C r = v0, i = cmk<C>(0, 0);
 #pragma unroll
       for (int m = 1; m <= H; ++m) {
         if (!((MASK >> m) & 1) && !((MASK >> (R - m)) & 1)) continue;
         const int j = (m * k) % R;
-        const Real cs = (Real)reg::rcos(R, j <= H ? j : R - j);
-        const Real sn = (Real)(j <= H ? reg::rsin(R, j) : -reg::rsin(R, R - j));
-        rx += a[m].x * cs;
-        ry += a[m].y * cs;
-        ix += b[m].x * sn;
-        iy += b[m].y * sn;
+        r = reg::cfma(a[m], (Real)reg::rcos(R, j <= H ? j : R - j), r);
+        i = reg::cfma(b[m], (Real)(j <= H ? reg::rsin(R, j) : -reg::rsin(R, R - j)), i);
       }
-      out[k] = cmk<C>(rx - DIR * iy, ry + DIR * ix);
-      out[R - k] = cmk<C>(rx + DIR * iy, ry - DIR * ix);
+      out[k] = cadd(r, i);
+      out[R - k] = csub(r, i);
     }
 #pragma unroll
     for (int k = 0; k < R; ++k) v[k] = out[k];
