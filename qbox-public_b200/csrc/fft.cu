@@ -1309,22 +1309,18 @@ void basis_ft_forward(Context& ctx, const DeviceSticks& d, int ng, bool real_bas
 // the GGA's last two fields packed into one transform, update_vhxc takes (ms)
 // 0.45 -> 0.22 at 84^3 and 1.24 -> 0.57 at 140^3, PBE; what is left there is
 // the latency of some twenty short kernels, and at 140^3 HBM.
-static pen::Args field_args(Context& ctx) {
-  const DeviceSticks& g = ctx.dvs;
-  pen::Args a;
-  a.g = g;
-  for (int i = 0; i < 3; i++) a.tw[i] = g.tw[i];
-  a.scale = 1.0 / (double)ctx.N();
-  a.ngw = ctx.vb.ng;
-  a.nslots = 1;
-  a.sticks = ctx.d_zfast;
-  a.tile = (double2*)ctx.d_zfast + (size_t)g.nvec * g.n2;
-  a.stream = ctx.stream;
-  return a;
-}
-static void field_passes(Context& ctx, pen::Args& a, bool back) {
+// Two transforms (the GGA's three gradient components) go through as two slots of
+// the same launches.
+static void field_passes(Context& ctx, pen::Args& a, int nslots, bool back) {
   ProfScope ps(ctx, "grid_fft");
   const DeviceSticks& g = ctx.dvs;
+  a.g = g;
+  for (int i = 0; i < 3; i++) a.tw[i] = g.tw[i];
+  a.ngw = ctx.vb.ng;
+  a.nslots = a.chunks = nslots;
+  a.sticks = ctx.d_zfast;
+  a.tile = (double2*)ctx.d_zfast + (size_t)nslots * g.nvec * g.n2;
+  a.stream = ctx.stream;
   const int order[3] = {back ? pen::GZB : pen::GXG, back ? pen::GYB : pen::GYF,
                         back ? pen::GXR : pen::GZF};
   const int n[3] = {back ? g.n2 : g.n0, g.n1, back ? g.n0 : g.n2};
@@ -1337,25 +1333,25 @@ static void field_passes(Context& ctx, pen::Args& a, bool back) {
 // c0 + i c1 (c1, f1 may be null)
 static void fields_backward(Context& ctx, const double* c0, const double* c1, double* f0,
                             double* f1, const double* add, bool chain) {
-  pen::Args a = field_args(ctx);
-  a.c = (const double2*)c0;
-  a.cb = (const double2*)c1;
-  a.f0 = f0;
-  a.f1 = f1;
+  pen::Args a;
+  a.gc[0] = (double2*)c0;
+  a.gc[1] = (double2*)c1;
+  a.gf[0] = f0;
+  a.gf[1] = f1;
   a.fadd = add;
   a.chain = chain;
-  field_passes(ctx, a, true);
+  field_passes(ctx, a, 1, true);
 }
 static void fields_forward(Context& ctx, const double* f0, const double* f1, const double* mul,
                            double scale, double* c0, double* c1) {
-  pen::Args a = field_args(ctx);
-  a.f0 = (double*)f0;
-  a.f1 = (double*)f1;
+  pen::Args a;
+  a.gf[0] = (double*)f0;
+  a.gf[1] = (double*)f1;
   a.fmul = mul;
-  a.scale *= scale;
-  a.hc = (double2*)c0;
-  a.hcb = (double2*)c1;
-  field_passes(ctx, a, false);
+  a.scale = scale / (double)ctx.N();
+  a.gc[0] = (double2*)c0;
+  a.gc[1] = (double2*)c1;
+  field_passes(ctx, a, 1, false);
 }
 
 void vb_backward(Context& ctx, const double* coef, double* real_out) {
@@ -1411,6 +1407,45 @@ void vb_forward_real(Context& ctx, const double* f, double scale, double* coef) 
   k_gather_sphere<<<nblk(ctx.vb.ng), 256, 0, ctx.stream>>>((const double2*)ctx.d_grid, ctx.dvs.ip,
                                                            ctx.vb.ng, 1.0 / (double)N, (double2*)coef);
   QBX_LAUNCHED(ctx);
+}
+
+// two slots of the density basis fit the stick buffer
+static bool two_field_slots(const Context& ctx) {
+  const DeviceSticks& g = ctx.dvs;
+  return ctx.grid_zfast && ctx.zfast_bytes >= 2 * sizeof(double2) * (size_t)g.n2 *
+                                                  ((size_t)g.nvec + (size_t)g.ncol * g.n1);
+}
+// three real fields f, f + N, f + 2 N of the coefficients c[0], c[1], c[2], and
+// the coefficients of the three fields times w
+void vb_backward3(Context& ctx, double* const c[3], double* f) {
+  const size_t N = ctx.N();
+  if (!two_field_slots(ctx)) {
+    vb_backward_pair(ctx, c[0], c[1], f, f + N);
+    vb_backward(ctx, c[2], f + 2 * N);
+    return;
+  }
+  pen::Args a;
+  for (int j = 0; j < 3; j++) {
+    a.gc[j] = (double2*)c[j];
+    a.gf[j] = f + j * N;
+  }
+  field_passes(ctx, a, 2, true);
+}
+void vb_forward_real3(Context& ctx, const double* f, const double* w, double* const c[3]) {
+  const size_t N = ctx.N();
+  if (!two_field_slots(ctx)) {
+    vb_forward_real_pair(ctx, f, f + N, w, c[0], c[1]);
+    vb_forward_real_pair(ctx, f + 2 * N, nullptr, w, c[2], nullptr);
+    return;
+  }
+  pen::Args a;
+  for (int j = 0; j < 3; j++) {
+    a.gc[j] = (double2*)c[j];
+    a.gf[j] = (double*)f + j * N;
+  }
+  a.fmul = w;
+  a.scale = 1.0 / (double)N;
+  field_passes(ctx, a, 2, false);
 }
 
 // out0 = add + back(a) and, with b, out1 = out0 + back(b): the sums over the

@@ -120,14 +120,13 @@ struct Args {
   double wunit = 1;              // the sums take the weights in this unit ...
   double wout = 1;               // ... and are added to rho times this, in FP64
   bool rho_set = false;          // store the density instead of adding (chunks == 1)
-  // real fields on a whole grid (the density basis, G* passes, one slot)
-  const double2* cb = nullptr;   // second coefficient array, or null
-  double2* hcb = nullptr;
-  double* f0 = nullptr;          // the real and imaginary fields; f1 may be null
-  double* f1 = nullptr;
-  const double* fadd = nullptr;  // GXR: f0 = Re + fadd; GXG: f0, f1 times fmul
+  // real fields on a whole grid (the density basis, G* passes): two coefficient
+  // arrays and two fields per slot, the second of each may be null
+  double2* gc[4] = {nullptr, nullptr, nullptr, nullptr};
+  double* gf[4] = {nullptr, nullptr, nullptr, nullptr};
+  const double* fadd = nullptr;  // GXR: field 0 = Re + fadd; GXG: the fields times fmul
   const double* fmul = nullptr;
-  bool chain = false;            // GXR: f1 = Im + the new f0
+  bool chain = false;            // GXR: field 1 = Im + the new field 0
   cudaStream_t stream = nullptr;
 };
 
@@ -191,8 +190,8 @@ zb(Args a) {
   const int slot = blockIdx.y;
   load_tw<C, N>(tw, a.tw[2]);
   const int b1 = K ? a.first + slot : 2 * (a.first + slot);
-  const double2* c1 = a.c + (size_t)b1 * a.ngw;
-  const double2* c2 = G ? a.cb : (!K && b1 + 1 < a.nst) ? c1 + a.ngw : nullptr;
+  const double2* c1 = G ? a.gc[2 * slot] : a.c + (size_t)b1 * a.ngw;
+  const double2* c2 = G ? a.gc[2 * slot + 1] : (!K && b1 + 1 < a.nst) ? c1 + a.ngw : nullptr;
   __syncthreads();
   {
     const int j = threadIdx.x % R2, line = threadIdx.x / R2, s = s0 + line;
@@ -308,16 +307,18 @@ zf(Args a) {
       const C M = sm[sn * ZS<N>::LINE + zm];
       // c1 = (Z(G) + conj Z(-G))/2, c2 = -i (Z(G) - conj Z(-G))/2
       const double px = P.x, py = P.y, mx = M.x, my = M.y;
-      a.hc[i1] = make_double2(kin * x.x + 0.5 * (px + mx) * a.scale,
-                              kin * x.y + 0.5 * (py - my) * a.scale);
+      const double2 u = make_double2(0.5 * (px + mx) * a.scale, 0.5 * (py - my) * a.scale);
+      const double2 w = make_double2(0.5 * (py + my) * a.scale, 0.5 * (mx - px) * a.scale);
       if (G) {
-        if (a.hcb)
-          a.hcb[ig] = make_double2(0.5 * (py + my) * a.scale, 0.5 * (mx - px) * a.scale);
-      } else if (two) {
-        const size_t i2 = i1 + a.ngw;
-        const double2 y = a.c[i2];
-        a.hc[i2] = make_double2(kin * y.x + 0.5 * (py + my) * a.scale,
-                                kin * y.y + 0.5 * (mx - px) * a.scale);
+        a.gc[2 * slot][ig] = u;
+        if (a.gc[2 * slot + 1]) a.gc[2 * slot + 1][ig] = w;
+      } else {
+        a.hc[i1] = make_double2(kin * x.x + u.x, kin * x.y + u.y);
+        if (two) {
+          const size_t i2 = i1 + a.ngw;
+          const double2 y = a.c[i2];
+          a.hc[i2] = make_double2(kin * y.x + w.x, kin * y.y + w.y);
+        }
       }
     }
   }
@@ -576,10 +577,10 @@ xv(Args a) {
   }
 }
 
-// One complex transform of real fields on the whole grid: the tile to f0 (and
-// f1), or back from them.  The pointwise work next to it rides along: f0 takes
-// fadd (v_xc += ...), f1 the new f0 (V = V_local + v_xc), the fields to be
-// transformed are multiplied by fmul.
+// One complex transform of real fields on the whole grid per slot: the tile to
+// the slot's fields 0 (and 1), or back from them.  The pointwise work next to it
+// rides along: field 0 takes fadd (v_xc += ...), field 1 the new field 0 (V =
+// V_local + v_xc), the fields to be transformed are multiplied by fmul.
 template <int N>
 __global__ void __launch_bounds__((lines<double, N>()) * fac(N).r1, (min_ctas<double, N, KXY>()))
 xr(Args a) {
@@ -595,7 +596,7 @@ xr(Args a) {
   load_tw<C, N>(tw, a.tw[0]);
   C v[R1];
   if (item < R2 && on) {
-    const C* in = (const C*)a.tile + line;
+    const C* in = (const C*)a.tile + (size_t)blockIdx.y * g.ncol * nl + line;
 #pragma unroll
     for (int q = 0; q < R1; ++q) {
       const int col = g.xcol[item + q * R2];
@@ -610,12 +611,13 @@ xr(Args a) {
 #pragma unroll
   for (int j = 0; j < R2; ++j) u[j] = sm[(item * R2 + j) * kLines + lane];
   lane::dft_reg<R2, +1>(u);
+  double *f0 = a.gf[2 * blockIdx.y], *f1 = a.gf[2 * blockIdx.y + 1];
 #pragma unroll
   for (int m = 0; m < R2; ++m) {
     const size_t p = (size_t)(item + m * R1) * nl + line;
     const double f = a.fadd ? u[m].x + a.fadd[p] : u[m].x;
-    a.f0[p] = f;
-    if (a.f1) a.f1[p] = a.chain ? u[m].y + f : u[m].y;
+    f0[p] = f;
+    if (f1) f1[p] = a.chain ? u[m].y + f : u[m].y;
   }
 }
 
@@ -634,11 +636,12 @@ xg(Args a) {
   load_tw<C, N>(tw, a.tw[0]);
   C u[R2];
   if (on) {
+    const double *f0 = a.gf[2 * blockIdx.y], *f1 = a.gf[2 * blockIdx.y + 1];
 #pragma unroll
     for (int m = 0; m < R2; ++m) {
       const size_t p = (size_t)(item + m * R1) * nl + line;
       const double w = a.fmul ? a.fmul[p] : 1.0;
-      u[m] = make_double2(a.f0[p] * w, a.f1 ? a.f1[p] * w : 0.0);
+      u[m] = make_double2(f0[p] * w, f1 ? f1[p] * w : 0.0);
     }
   }
   __syncthreads();
@@ -649,7 +652,7 @@ xg(Args a) {
 #pragma unroll
     for (int k = 0; k < R1; ++k) v[k] = sm[(k * R2 + item) * kLines + lane];
     lane::dft_reg<R1, -1>(v);
-    C* out = (C*)a.tile + line;
+    C* out = (C*)a.tile + (size_t)blockIdx.y * g.ncol * nl + line;
 #pragma unroll
     for (int q = 0; q < R1; ++q) {
       const int col = g.xcol[item + q * R2];
@@ -766,7 +769,7 @@ void run(Context& ctx, const Args& a) {
         if (a.op == ZBK) zb<T, N, true><<<gzb, th, 0, st>>>(a);
         else if (a.op == ZFK) zf<T, N, true><<<dim3(cdiv(g.nrods, kLines), a.nslots), th, 0, st>>>(a);
         else if (a.op == GZB) zb<T, N, false, true><<<gzb, th, 0, st>>>(a);
-        else if (a.op == GZF) zf<T, N, false, true><<<cdiv(g.nrods, kLines / 2), th, 0, st>>>(a);
+        else if (a.op == GZF) zf<T, N, false, true><<<dim3(cdiv(g.nrods, kLines / 2), a.nslots), th, 0, st>>>(a);
         else if (a.op == GYB) yb<T, N, true><<<gy, th, 0, st>>>(a);
         else if (a.op == GYF) yf<T, N, true><<<gy, th, 0, st>>>(a);
         else if (a.op == GXR) xr<N><<<gx, th, 0, st>>>(a);

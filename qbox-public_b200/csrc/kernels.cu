@@ -137,12 +137,16 @@ __global__ void k_pbe(const double* __restrict__ rho, const double* __restrict__
 }
 
 // out(G) = i gx_j(G) scale in(G)
-__global__ void k_mul_igx(const double2* __restrict__ in, const double* __restrict__ gxj, int ng,
-                          double scale, double2* __restrict__ out) {
+// out_j = i G_j in scale for the three components (gx: x, y and z blocks of ng)
+__global__ void k_mul_igx3(const double2* __restrict__ in, const double* __restrict__ gx, int ng,
+                           double scale, double2* __restrict__ out) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ng; i += gridDim.x * blockDim.x) {
     const double2 v = in[i];
-    const double g = gxj[i] * scale;
-    out[i] = make_double2(-g * v.y, g * v.x);
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      const double g = gx[(size_t)j * ng + i] * scale;
+      out[(size_t)j * ng + i] = make_double2(-g * v.y, g * v.x);
+    }
   }
 }
 
@@ -196,14 +200,10 @@ void launch_xc(Context& ctx) {
   // components packed into one complex transform
   const int ngv = ctx.vb.ng;
   double* xg[3] = {ctx.d_xc_g, ctx.d_xc_g + 2 * (size_t)ngv, ctx.d_xc_g + 4 * (size_t)ngv};
-  for (int j = 0; j < 3; j++) {
-    k_mul_igx<<<blocks_for(ngv), kThreads, 0, ctx.stream>>>(
-        (const double2*)ctx.d_rhog, ctx.d_gx_v + (size_t)j * ngv, ngv, 1.0 / om,
-        (double2*)xg[j]);
-    QBX_LAUNCHED(ctx);
-  }
-  vb_backward_pair(ctx, xg[0], xg[1], ctx.d_grad, ctx.d_grad + N);
-  vb_backward(ctx, xg[2], ctx.d_grad + 2 * N);
+  k_mul_igx3<<<blocks_for(ngv), kThreads, 0, ctx.stream>>>(
+      (const double2*)ctx.d_rhog, ctx.d_gx_v, ngv, 1.0 / om, (double2*)ctx.d_xc_g);
+  QBX_LAUNCHED(ctx);
+  vb_backward3(ctx, xg, ctx.d_grad);
   k_pbe<<<nb, kThreads, 0, ctx.stream>>>(ctx.d_rhor, ctx.d_grad, N, ctx.d_vxc, ctx.d_vx2,
                                          ctx.d_exc);
   QBX_LAUNCHED(ctx);
@@ -211,8 +211,7 @@ void launch_xc(Context& ctx) {
   reduce<2>(ctx, SumRhoV1F{ctx.d_exc, ctx.d_rhor, ctx.d_vxc}, N, SLOT_EXC);
   // the divergence term sum_j i G_j forward(grad_j vxc2) in G space, two real
   // fields to a complex transform; launch_vhxc_rspace takes it back to r
-  vb_forward_real_pair(ctx, ctx.d_grad, ctx.d_grad + N, ctx.d_vx2, xg[0], xg[1]);
-  vb_forward_real_pair(ctx, ctx.d_grad + 2 * N, nullptr, ctx.d_vx2, xg[2], nullptr);
+  vb_forward_real3(ctx, ctx.d_grad, ctx.d_vx2, xg);
   k_sum_igx3<<<blocks_for(ngv), kThreads, 0, ctx.stream>>>(
       (const double2*)xg[0], (const double2*)xg[1], (const double2*)xg[2], ctx.d_gx_v, ngv,
       (double2*)ctx.d_vtmp_g);

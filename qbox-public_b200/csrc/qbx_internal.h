@@ -600,6 +600,9 @@ void vb_backward_add(Context& ctx, const double* a, const double* b, const doubl
                      double* out0, double* out1);
 // whether the grids can be kept z fastest, and their conversion from and to
 // the callers' x-fastest order (device arrays)
+// three real fields f, f + N, f + 2 N from and (times w) to their coefficients
+void vb_backward3(Context& ctx, double* const c[3], double* f);
+void vb_forward_real3(Context& ctx, const double* f, const double* w, double* const c[3]);
 bool grid_zfast_possible(const Context& ctx);
 void kpoints_grid_order(Context& ctx);   // after the set of k points changed
 void grid_to_caller(Context& ctx, const double* f, double* out);
