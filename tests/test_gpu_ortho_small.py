@@ -78,3 +78,18 @@ def test_singular_overlap_is_an_error(precision):
     np.testing.assert_allclose(ctx.get_coeffs(), c, rtol=0,
                                atol=1e-11 if precision == capi.FP64 else 1e-6)
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 65, 200, 432])
+def test_lower_inverse_with_smaller_last_blocks(n):
+    """L^-1 by blocks whose last ones are not whole: n eps times the factor's
+    condition number (4)."""
+    rng = np.random.default_rng(n)
+    l = np.tril(0.5 / np.sqrt(n) * rng.standard_normal((n, n)), -1) + np.diag(rng.uniform(1, 2, n))
+    bad = l.copy()
+    bad[np.triu_indices(n, 1)] = np.nan
+    ctx = _ctx(4, capi.MIXED, "1")
+    got, _ = ctx.lower_inverse(bad)
+    np.testing.assert_allclose(got @ l, np.eye(n), rtol=0, atol=64 * n * np.finfo(float).eps)
+    assert np.all(got[np.triu_indices(n, 1)] == 0.0)
+    ctx.close()
