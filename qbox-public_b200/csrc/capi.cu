@@ -442,6 +442,9 @@ void qbx_destroy(qbx_context* h) {
   dfree(h->d_perm);
   dfree(h->c.d_status);
   if (h->c.d_blas_ws) cudaFree(h->c.d_blas_ws);
+  if (h->c.h_stage) cudaFreeHost(h->c.h_stage);
+  for (cudaEvent_t e : h->c.ev_stage)
+    if (e) cudaEventDestroy(e);
   if (h->c.h_scalars) cudaFreeHost(h->c.h_scalars);
   if (h->c.h_status) cudaFreeHost(h->c.h_status);
   if (h->c.blas) cublasDestroy(h->c.blas);
@@ -1406,11 +1409,56 @@ void upload_wf(qbx_context* h, const double* src, double* dst) {
   }
 }
 
-// device (internal order) -> host vector (caller order)
-std::vector<double> download_wf(qbx_context* h, const double* dsrc) {
+// dst[i] += scale * src[i], src on the device (all of it written by work already
+// on c.stream), dst the caller's array.  1 MB pieces through pinned slots of the
+// context, each slot served by a thread that waits for its copy and adds it, so
+// that the copies run on while the additions, which the host's memory bounds,
+// are spread over the threads.  (Into a fresh vector and added by one thread,
+// 20 MB took 7 ms, most of it page faults and the addition.)
+void add_to_caller(Context& c, const double* src, size_t n, double scale, double* dst) {
+  constexpr size_t kPiece = (size_t)1 << 17;
+  const size_t pieces = (n + kPiece - 1) / kPiece;
+  const size_t most = std::max(1u, std::thread::hardware_concurrency() / 2);
+  const int nt = (int)std::min({pieces, (size_t)Context::kStageSlots, most});
+  if (!c.h_stage)
+    QBX_CUDA(cudaMallocHost(&c.h_stage, Context::kStageSlots * kPiece * sizeof(double)));
+  for (int t = 0; t < nt; t++) {
+    if (!c.ev_stage[t]) QBX_CUDA(cudaEventCreateWithFlags(&c.ev_stage[t], cudaEventDisableTiming));
+  }
+  std::atomic<int> failed{0};
+  auto serve = [&](int t) {
+    if (cudaSetDevice(c.device) != cudaSuccess) failed = 1;
+    for (size_t i = t; i < pieces && !failed; i += nt) {
+      const size_t off = i * kPiece, m = std::min(kPiece, n - off);
+      double* buf = c.h_stage + t * kPiece;
+      if (cudaMemcpyAsync(buf, src + off, m * sizeof(double), cudaMemcpyDeviceToHost,
+                          c.stream) != cudaSuccess ||
+          cudaEventRecord(c.ev_stage[t], c.stream) != cudaSuccess ||
+          cudaEventSynchronize(c.ev_stage[t]) != cudaSuccess) {
+        failed = 1;
+        break;
+      }
+      double* d = dst + off;
+      for (size_t k = 0; k < m; k++) d[k] += scale * buf[k];
+    }
+  };
+  std::vector<std::thread> others;
+  int served = 1;                    // slots whose pieces someone serves
+  try {
+    for (; served < nt; served++) others.emplace_back(serve, served);
+  } catch (const std::exception&) {
+    // no thread to be had: this one serves the rest
+  }
+  serve(0);
+  for (int t = served; t < nt; t++) serve(t);
+  for (std::thread& t : others) t.join();
+  QBX_REQUIRE(!failed, 2, std::string("copy to the caller's array: ") +
+                              cudaGetErrorString(cudaGetLastError()));
+}
+
+// a wavefunction block (internal order) added to the caller's (its order)
+void add_wf_to_caller(qbx_context* h, const double* dsrc, double* dst) {
   Context& c = h->c;
-  const size_t wf = 2 * (size_t)c.wb.ng * c.nst;
-  std::vector<double> out(wf);
   const double* src = dsrc;
   if (h->d_perm) {
     k_permute<<<1184, 256, 0, c.stream>>>((const double2*)dsrc, h->d_perm, c.wb.ng, c.nst, 0,
@@ -1418,9 +1466,7 @@ std::vector<double> download_wf(qbx_context* h, const double* dsrc) {
     QBX_LAUNCHED(c);
     src = c.d_ctmp;
   }
-  QBX_CUDA(cudaMemcpyAsync(out.data(), src, wf * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-  QBX_CUDA(cudaStreamSynchronize(c.stream));
-  return out;
+  add_to_caller(c, src, 2 * (size_t)c.wb.ng * c.nst, 1.0, dst);
 }
 
 }  // namespace
@@ -1433,11 +1479,7 @@ int qbx_compute_density(qbx_context* h, double weight, double* rho) {
     const size_t N = c.N();
     if (!c.d_xgrid) c.d_xgrid = dalloc<double>(N);
     launch_density(c, c.d_c, c.d_xgrid);
-    std::vector<double> tmp(N);
-    QBX_CUDA(cudaMemcpyAsync(tmp.data(), caller_grid(c, c.d_xgrid), N * sizeof(double),
-                             cudaMemcpyDeviceToHost, c.stream));
-    QBX_CUDA(cudaStreamSynchronize(c.stream));
-    for (size_t i = 0; i < N; i++) rho[i] += weight * tmp[i];
+    add_to_caller(c, caller_grid(c, c.d_xgrid), N, weight, rho);
   });
 }
 
@@ -1456,8 +1498,7 @@ int qbx_rs_mul_add(qbx_context* h, const double* v, double* dc) {
     k_sub_kinetic<<<1184, 256, 0, c.stream>>>((double2*)out, (const double2*)c.d_c, c.d_g2_w,
                                               c.wb.ng, c.nst);
     QBX_LAUNCHED(c);
-    const std::vector<double> add = download_wf(h, out);
-    for (size_t i = 0; i < add.size(); i++) dc[i] += add[i];
+    add_wf_to_caller(h, out, dc);
   });
 }
 
@@ -1484,10 +1525,7 @@ int qbx_nonlocal_energy(qbx_context* h, int compute_hpsi, double* dc, int comput
     if (enl) *enl = e_nl;
     if (compute_forces) std::memcpy(fion, c.h_fion, sizeof(double) * 3 * natoms);
     if (compute_stress) nl_stress_part(c, e_nl, sigma_enl);
-    if (compute_hpsi) {
-      const std::vector<double> add = download_wf(h, out);
-      for (size_t i = 0; i < add.size(); i++) dc[i] += add[i];
-    }
+    if (compute_hpsi) add_wf_to_caller(h, out, dc);
   });
 }
 

@@ -515,6 +515,11 @@ struct Context {
   bool in_pending = false;       // an upload not yet consumed by a step
   bool finish_pending = false;   // a captured step whose host finish is deferred
   double last_energies[16] = {0};
+  // pinned 1 MB pieces through which the class-level entry points add to the
+  // caller's arrays, allocated on first use
+  static constexpr int kStageSlots = 6;
+  double* h_stage = nullptr;
+  cudaEvent_t ev_stage[kStageSlots] = {nullptr};
   // k points off Gamma; when set, the electronic step runs on them instead
   // of the Gamma coefficients
   std::vector<KPointSet> kpts;
@@ -595,14 +600,14 @@ void vb_backward_pair(Context& ctx, const double* a, const double* b, double* ou
 // transform, with the 1/N of the forward transform
 void vb_forward_real_pair(Context& ctx, const double* f0, const double* f1, const double* w,
                           double* c0, double* c1);
+// three real fields f, f + N, f + 2 N from and (times w) to their coefficients
+void vb_backward3(Context& ctx, double* const c[3], double* f);
+void vb_forward_real3(Context& ctx, const double* f, const double* w, double* const c[3]);
 // out0 = add + back(a); with b also out1 = out0 + back(b) (d_exc is scratch)
 void vb_backward_add(Context& ctx, const double* a, const double* b, const double* add,
                      double* out0, double* out1);
 // whether the grids can be kept z fastest, and their conversion from and to
 // the callers' x-fastest order (device arrays)
-// three real fields f, f + N, f + 2 N from and (times w) to their coefficients
-void vb_backward3(Context& ctx, double* const c[3], double* f);
-void vb_forward_real3(Context& ctx, const double* f, const double* w, double* const c[3]);
 bool grid_zfast_possible(const Context& ctx);
 void kpoints_grid_order(Context& ctx);   // after the set of k points changed
 void grid_to_caller(Context& ctx, const double* f, double* out);
