@@ -17,12 +17,15 @@
 //   polar:  X <- polar(X)
 //
 // What bounds it: the serial chain of pivots in the Cholesky factor (one warp per
-// 16 x 16 diagonal block), then the latency of a product's operand copy from L2
-// and of the cluster barriers.  16 bands 24 us, 128 bands 155 us; psda_update of
-// the eager step (ms) at 16 bands FP64 0.38 -> 0.17, 97 bands mixed 0.60 -> 0.34,
-// 128 bands mixed 0.63 -> 0.42.  The limit of 128 is one matrix in a CTA's shared
+// 16 x 16 diagonal block, its rows in registers: 95 of 155 us at 128 bands before
+// every index of them was a compile-time one), then the latency of a product's
+// operand copy from L2 and of the cluster barriers.  16 bands 22 us, 128 bands 109
+// us; psda_update of the eager step (ms) at 16 bands FP64 0.38 -> 0.13, 97 bands
+// mixed 0.60 -> 0.30, 128 bands mixed 0.63 -> 0.38 (FP64 with the whole-product
+// overlap 0.92 -> 0.40).  The limit of 128 is one matrix in a CTA's shared
 // memory and eight panels in a portable cluster.
 #include <cstdint>
+#include <type_traits>
 
 #include "qbx_internal.h"
 
@@ -135,6 +138,29 @@ __device__ __forceinline__ void panel_mm(const double* A, const double* B, int n
   }
 }
 
+// f(0) ... f(E - 1) with compile-time indices (rows held in registers)
+template <int I, int E, typename F> __device__ __forceinline__ void unroll(const F& f) {
+  if constexpr (I < E) {
+    f(std::integral_constant<int, I>{});
+    unroll<I + 1, E>(f);
+  }
+}
+
+// 1/sqrt(d) for a pivot: an FP32 estimate and two Newton steps y += y (1 - d y^2)/2,
+// each doubling its 23 bits (the pivots form one serial chain, where the library
+// function's handling of every exponent costs as much again); pivots beyond the
+// FP32 range take the library function.
+__device__ __forceinline__ double pivot_rsqrt(double d) {
+  if (!(d > 1e-30 && d < 1e30)) return rsqrt(d);
+  double y = (double)rsqrtf((float)d);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const double e = fma(-d * y, y, 1.0);
+    y = fma(0.5 * y, e, y);
+  }
+  return y;
+}
+
 // A (np x np in shared memory, lower triangle of an SPD matrix) <- inverse of
 // its Cholesky factor, strictly upper triangle zero.  16-column panels: the
 // diagonal block by one warp, the rest by MMAs.  Returns 0, or the order of the
@@ -150,38 +176,35 @@ __device__ int cholesky_inverse(double* A, double* tmp, double* dia, int np, dou
       double row[16], inv = 0.0;   // row i of the block, 1 / L_ii
 #pragma unroll
       for (int k = 0; k < 16; ++k) row[k] = A[(p + k) * P + p + i];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
+      unroll<0, 16>([&](auto j) {
         double d = __shfl_sync(0xffffffffu, row[j], j);
         if (!(d > 0.0)) {
           if (lane == 0 && flag[0] == 0.0) flag[0] = p + j + 1;
           d = 1.0;
         }
-        const double si = rsqrt(d), s = d * si;   // the chain of pivots is serial
-        row[j] = i == j ? s : row[j] * si;
+        const double si = pivot_rsqrt(d);
         if (i == j) inv = si;
-#pragma unroll
-        for (int k = j + 1; k < 16; ++k) {
+        row[j] = i == j ? d * si : row[j] * si;
+        unroll<decltype(j)::value + 1, 16>([&](auto k) {
           const double l = __shfl_sync(0xffffffffu, row[j], k);
           if (i >= k) row[k] -= row[j] * l;
-        }
-      }
+        });
+      });
       __syncwarp();
       if (lane < 16) {
 #pragma unroll
         for (int k = 0; k < 16; ++k) A[(p + k) * P + p + i] = k <= i ? row[k] : 0.0;
       }
       __syncwarp();
-      // column i of the inverse by forward substitution
+      // column i of the inverse by forward substitution, each x_r taken out of
+      // all later rows at once
       double x[16];
 #pragma unroll
-      for (int r = 0; r < 16; ++r) {
-        double s = r == i ? 1.0 : 0.0;
-#pragma unroll
-        for (int k = 0; k < r; ++k) s -= A[(p + k) * P + p + r] * x[k];
-        const double ir = __shfl_sync(0xffffffffu, inv, r);
-        x[r] = r < i ? 0.0 : s * ir;
-      }
+      for (int r = 0; r < 16; ++r) x[r] = r == i ? 1.0 : 0.0;
+      unroll<0, 16>([&](auto r) {
+        x[r] *= __shfl_sync(0xffffffffu, inv, r);
+        unroll<decltype(r)::value + 1, 16>([&](auto k) { x[k] -= A[(p + r) * P + p + k] * x[r]; });
+      });
       __syncwarp();
       if (lane < 16) {
 #pragma unroll
@@ -189,27 +212,36 @@ __device__ int cholesky_inverse(double* A, double* tmp, double* dia, int np, dou
       }
     }
     __syncthreads();
-    // L21 = A21 L11^-T; the inverse block waits in place of L11
+    // L21 = A21 L11^-T in place, 16 rows a warp; the inverse block waits in place
+    // of L11
     const int below = np - p - 16;
-    for (int t = threadIdx.x; t < below * 16; t += kThreads) {
-      const int c = t / below, r = p + 16 + t - c * below;
-      double s = 0.0;
-      for (int k = 0; k <= c; ++k) s += A[(p + k) * P + r] * dia[c * 20 + k];
-      tmp[c * P + r] = s;
+    const int lr = lane >> 2, lk = lane & 3, lc = 2 * lk;
+    if (16 * warp < below) {
+      double c[2][2][2] = {};
+      const int r0 = p + 16 + 16 * warp;
+#pragma unroll
+      for (int k = 0; k < 16; k += 4) {
+        double a[2], b[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          a[h] = A[(p + k + lk) * P + r0 + 8 * h + lr];
+          b[h] = dia[(8 * h + lr) * 20 + k + lk];
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int g = 0; g < 2; ++g) dmma(c[h][g], a[h], b[g]);
+      }
+      __syncwarp();
+      each(c, r0, [&](int r, int cc, double v) { A[(p + cc) * P + r] = v; });
     }
-    __syncthreads();
-    for (int t = threadIdx.x; t < below * 16; t += kThreads) {
-      const int c = t / below, r = p + 16 + t - c * below;
-      A[(p + c) * P + r] = tmp[c * P + r];
-    }
-    if (threadIdx.x < 256) {
+    {
       const int c = threadIdx.x >> 4, r = threadIdx.x & 15;
       A[(p + c) * P + p + r] = r >= c ? dia[r * 20 + c] : 0.0;
     }
     __syncthreads();
     // A22 -= L21 L21^T, lower 8 x 8 tiles
     const int nt = below / 8;
-    const int lr = lane >> 2, lk = lane & 3, lc = 2 * lk;
     for (int t = warp; t < nt * nt; t += 8) {
       const int ti = t / nt, tj = t - ti * nt;
       if (tj > ti) continue;
@@ -228,24 +260,22 @@ __device__ int cholesky_inverse(double* A, double* tmp, double* dia, int np, dou
   for (int p = np - 32; p >= 0; p -= 16) {
     const int below = np - p - 16;
     const int row0 = 16 * warp;
+    double d[2][2][2] = {};
     if (row0 < below) {
       double c[2][2][2] = {};
       warp_mm<false>(A + (p + 16) * P + p + 16, A + p * P + p + 16, row0, row0 + 16, c);
-      each(c, row0, [&](int r, int cc, double v) { tmp[cc * P + r] = v; });
+      each(c, row0, [&](int r, int cc, double v) { tmp[cc * P + r] = -v; });
+      __syncwarp();
+      warp_mm<false>(tmp, A + p * P + p, row0, 16, d);
     }
-    __syncthreads();
-    for (int t = threadIdx.x; t < below * 16; t += kThreads) {
-      const int c = t / below, r = t - c * below;
-      double s = 0.0;
-      for (int k = c; k < 16; ++k) s += tmp[k * P + r] * A[(p + c) * P + p + k];
-      A[(p + c) * P + p + 16 + r] = -s;
-    }
+    __syncthreads();                 // every warp has read the old column block
+    if (row0 < below)
+      each(d, row0, [&](int r, int cc, double v) { A[(p + cc) * P + p + 16 + r] = v; });
     __syncthreads();
   }
-  for (int t = threadIdx.x; t < np * np; t += kThreads) {
-    const int c = t / np, r = t - c * np;
-    if (r < c) A[c * P + r] = 0.0;
-  }
+  const int zr = threadIdx.x & (kMax - 1);
+  for (int c = threadIdx.x / kMax; c < np; c += kThreads / kMax)
+    if (zr < c) A[c * P + zr] = 0.0;
   __syncthreads();
   return (int)flag[0];
 }
