@@ -1,31 +1,18 @@
 // Staged 3-D FFTs of the electronic step on sm_100a.
 //
-// Wavefunction transforms (the hot path) never build the full 3-D grid in
-// HBM.  A band pair psi_1 + i psi_2 (the reference's two-real-functions
-// packing, src/BasisMapping.cpp:667-750) goes through three kernels:
+// Wavefunction transforms (the hot path) never build the full 3-D grid in HBM.  A
+// band pair psi_1 + i psi_2 (the reference's two-real-functions packing,
+// src/BasisMapping.cpp:667-750), or a band at a k point, goes through z sticks,
+// y columns and x rows; the density sum and the product with V(r) happen in the
+// x pass.  The kernels are the line passes of fft_pencil.cuh; this file holds their
+// launches (pencil_pass), the density-basis transforms on the same kernels
+// (field_passes), and the runtime-radix kernels for what those do not take:
 //
-//   k_zfft_bwd : gather the coefficients of a few rods, expand them into
-//                z-sticks (+G and -G columns), inverse FFT along z in shared
-//                memory, write the sticks plane-major  zbuf[pair][z][stick].
-//   k_xy       : one CTA per z-plane: scatter that plane's stick values into
-//                a compact (x-column x y) tile in shared memory, inverse FFT
-//                along y on the occupied columns only, then row by row the
-//                inverse FFT along x, and the fused real-space operation:
-//                  OP_DENSITY: rho += f1/Omega psi_1^2 + f2/Omega psi_2^2
-//                  OP_VPSI:    psi *= V(r), forward x FFT, back into the tile;
-//                              forward y FFT, write the plane's sticks back.
-//   k_zfft_fwd : forward z FFT of the sticks, unpack the two bands
-//                (src/BasisMapping.cpp:722-750), scale by 1/N and write
-//                hc = 1/2|G|^2 c + result   (kinetic term fused).
-//
-// Per band pair the HBM traffic is the coefficients, the sticks written and
-// read in each direction and the potential plane: the staged floor.
-//
-// Density-basis transforms (a handful per step) use the full grid with three
-// strided line-FFT passes (k_line_fft).
-//
-// All 1-D FFTs are mixed-radix (2,3,4,5,7,11) self-sorting Stockham passes
-// over shared memory with a twiddle table exp(+2 pi i k/n) built in FP64.
+//   k_zfft_bwd, k_xy, k_zfft_fwd : one CTA per z plane, mixed-radix (2, 3, 4, 5, 7,
+//                11) self-sorting Stockham passes over shared memory with a twiddle
+//                table exp(+2 pi i k/n) built in FP64: grids with a length above
+//                256, and qbx_density_static
+//   k_line_fft : the lines of a whole grid, the same passes
 #include <algorithm>
 #include <complex>
 #include <cstdio>

@@ -34,9 +34,9 @@
 // for every other grid and for k points, runtime-radix kernels.  What bounds
 // them now is HBM for the y passes (80 % of the measured copy rate at 140^3)
 // and FP32 issue with the shared-memory exchange for xv.  Per step, density +
-// H psi, before and after (ms): 512 atoms 140^3 FP32 15.5 -> 12.3, FP64 94.7 ->
-// 24.0; 64 atoms 84^3 FP32 0.70 -> 0.45, FP64 2.24 -> 0.71; 112 x 72 x 40 FP32
-// 1.09 -> 0.27; two k points 84^3 FP64 13.4 -> 2.5.
+// H psi, before and after (ms): 512 atoms 140^3 FP32 15.5 -> 10.6, FP64 94.7 ->
+// 21.1; 64 atoms 84^3 FP32 0.70 -> 0.40, FP64 2.24 -> 0.67; 112 x 72 x 40 FP32
+// 1.09 -> 0.23; two k points 84^3 FP64 13.4 -> 2.4.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -130,11 +130,15 @@ struct Args {
   cudaStream_t stream = nullptr;
 };
 
+// the twiddles W_N^{jk} as [k][j]: a thread's j or k is fixed, so every twiddle
+// it reads lies at a constant offset from its first (with the x passes' column
+// offsets kept as products: xv at 140^3 FP32 4.06 -> 3.57 ms, FP64 8.5 -> 7.5)
 template <typename C, int N>
 __device__ __forceinline__ void load_tw(C* tw, const double2* src) {
-  for (int k = threadIdx.x; k < N; k += blockDim.x) {
-    const double2 w = __ldg(src + k);
-    tw[k] = cmk<C>(w.x, w.y);
+  constexpr int R2 = fac(N).r2;
+  for (int i = threadIdx.x; i < N; i += blockDim.x) {
+    const double2 w = __ldg(src + (i / R2) * (i % R2));
+    tw[i] = cmk<C>(w.x, w.y);
   }
 }
 
@@ -142,13 +146,14 @@ __device__ __forceinline__ void load_tw(C* tw, const double2* src) {
 // shared memory at [k][j] (strides sk, sj)
 template <int N, int DIR, bool ALL = false, typename C>
 __device__ __forceinline__ void first_half(C (&v)[fac(N).r1], int j, const C* tw, C* s, int sk) {
-  constexpr int R1 = fac(N).r1;
+  constexpr int R1 = fac(N).r1, R2 = fac(N).r2;
   constexpr unsigned MASK = Keep<N>::template mask<ALL>();
   lane::dft_reg_in<R1, DIR, MASK>(v);
   s[0] = v[0];
+  tw += j;
 #pragma unroll
   for (int k = 1; k < R1; ++k) {
-    const C w = tw[j * k];
+    const C w = tw[k * R2];
     s[k * sk] = DIR > 0 ? cmul(v[k], w) : cmulc(v[k], w);
   }
 }
@@ -159,9 +164,10 @@ __device__ __forceinline__ void first_half_rev(C (&u)[fac(N).r2], int k, const C
   constexpr int R2 = fac(N).r2;
   lane::dft_reg<R2, DIR>(u);
   s[0] = u[0];
+  tw += k * R2;
 #pragma unroll
   for (int j = 1; j < R2; ++j) {
-    const C w = tw[j * k];
+    const C w = tw[j];
     s[j * sj] = DIR > 0 ? cmul(u[j], w) : cmulc(u[j], w);
   }
 }
@@ -188,18 +194,17 @@ zb(Args a) {
   const DeviceSticks& g = a.g;
   const int s0 = blockIdx.x * kLines;
   const int slot = blockIdx.y;
-  load_tw<C, N>(tw, a.tw[2]);
   const int b1 = K ? a.first + slot : 2 * (a.first + slot);
   const double2* c1 = G ? a.gc[2 * slot] : a.c + (size_t)b1 * a.ngw;
   const double2* c2 = G ? a.gc[2 * slot + 1] : (!K && b1 + 1 < a.nst) ? c1 + a.ngw : nullptr;
-  __syncthreads();
   {
     const int j = threadIdx.x % R2, line = threadIdx.x / R2, s = s0 + line;
-    if (line < kLines && s < g.nvec) {
+    const bool on = line < kLines && s < g.nvec;
+    C v[R1];
+    if (on) {
       const int r = K ? s : (s + 1) >> 1;
       const int lmin = g.rod_lmin[r], size = g.rod_size[r], first = g.rod_first[r];
       const bool mstick = !K && s > 0 && (s & 1) == 0;
-      C v[R1];
 #pragma unroll
       for (int q = 0; q < R1; ++q) {
         v[q] = cmk<C>(0, 0);
@@ -220,8 +225,10 @@ zb(Args a) {
           }
         }
       }
-      first_half<N, +1, G>(v, j, tw, sm + line * ZS<N>::LINE + j, ZS<N>::PJ);
     }
+    load_tw<C, N>(tw, a.tw[2]);        // while the coefficients arrive
+    __syncthreads();
+    if (on) first_half<N, +1, G>(v, j, tw, sm + line * ZS<N>::LINE + j, ZS<N>::PJ);
   }
   __syncthreads();
   const int k = threadIdx.x % R1, line = threadIdx.x / R1, s = s0 + line;
@@ -253,17 +260,18 @@ zf(Args a) {
   const int s0 = K ? r0 : (r0 == 0 ? 0 : 2 * r0 - 1);
   const int nl = (K ? r1 : 2 * r1 - 1) - s0;
   const int slot = blockIdx.y;
-  load_tw<C, N>(tw, a.tw[2]);
-  __syncthreads();
   {
     const int k = threadIdx.x % R1, line = threadIdx.x / R1;
+    C u[R2];
     if (line < nl) {
       const C* in = (const C*)a.sticks + ((size_t)slot * g.nvec + s0 + line) * N + k;
-      C u[R2];
 #pragma unroll
       for (int m = 0; m < R2; ++m) u[m] = in[m * R1];
-      first_half_rev<N, -1>(u, k, tw, sm + line * ZS<N>::LINE + k * ZS<N>::PJ, 1);
     }
+    load_tw<C, N>(tw, a.tw[2]);        // while the sticks arrive
+    __syncthreads();
+    if (line < nl)
+      first_half_rev<N, -1>(u, k, tw, sm + line * ZS<N>::LINE + k * ZS<N>::PJ, 1);
   }
   __syncthreads();
   {
@@ -441,11 +449,15 @@ yf(Args a) {
 // a register until the chunk ends, and V(r) is read once.  The next slot's
 // loads are in flight over the second half.
 template <int N>
-__device__ __forceinline__ void x_columns(const DeviceSticks& g, int item, int (&col)[fac(N).r1]) {
+__device__ __forceinline__ void x_columns(const DeviceSticks& g, int item, int nl,
+                                          int (&off)[fac(N).r1]) {
   constexpr int R1 = fac(N).r1, R2 = fac(N).r2;
 #pragma unroll
   for (int q = 0; q < R1; ++q)
-    if (Keep<N>::q(q)) col[q] = g.xcol[item + q * R2];
+    if (Keep<N>::q(q)) {
+      const int col = g.xcol[item + q * R2];
+      off[q] = col < 0 ? -1 : col * nl;
+    }
 }
 
 template <typename T, int N>
@@ -461,8 +473,8 @@ xd(Args a) {
   const int nl = g.n1 * g.n2;
   const bool on = line < nl;
   load_tw<C, N>(tw, a.tw[0]);
-  int col[R1];
-  if (item < R2) x_columns<N>(g, item, col);
+  int off[R1];
+  if (item < R2) x_columns<N>(g, item, nl, off);
   T acc[R2];
 #pragma unroll
   for (int m = 0; m < R2; ++m) acc[m] = 0;
@@ -476,7 +488,7 @@ xd(Args a) {
 #pragma unroll
     for (int q = 0; q < R1; ++q) {
       v[q] = cmk<C>(0, 0);
-      if (Keep<N>::q(q) && col[q] >= 0) v[q] = in[(size_t)col[q] * nl];
+      if (Keep<N>::q(q) && off[q] >= 0) v[q] = in[off[q]];
     }
   };
   int slot = blockIdx.y * per;
@@ -529,8 +541,8 @@ xv(Args a) {
   const int nl = g.n1 * g.n2;
   const bool on = line < nl, load = item < R2 && on;
   load_tw<C, N>(tw, a.tw[0]);
-  int col[R1];
-  if (item < R2) x_columns<N>(g, item, col);
+  int off[R1];
+  if (item < R2) x_columns<N>(g, item, nl, off);
   T vr[R2];
   if (on) {
     const T* v = (const T*)a.v + (size_t)item * nl + line;
@@ -548,7 +560,7 @@ xv(Args a) {
 #pragma unroll
       for (int q = 0; q < R1; ++q) {
         v[q] = cmk<C>(0, 0);
-        if (Keep<N>::q(q) && col[q] >= 0) v[q] = tile[(size_t)col[q] * nl];
+        if (Keep<N>::q(q) && off[q] >= 0) v[q] = tile[off[q]];
       }
       first_half<N, +1>(v, item, tw, sm + item * kLines + lane, R2 * kLines);
     }
@@ -572,7 +584,7 @@ xv(Args a) {
       lane::dft_reg<R1, -1>(v);
 #pragma unroll
       for (int q = 0; q < R1; ++q)
-        if (Keep<N>::q(q) && col[q] >= 0) tile[(size_t)col[q] * nl] = v[q];
+        if (Keep<N>::q(q) && off[q] >= 0) tile[off[q]] = v[q];
     }
   }
 }
