@@ -527,7 +527,19 @@ xd(Args a) {
 // The tile in place: x transform to psi(r), times V(r), transform back.  A
 // thread's second-half reads and its writes of the way back are the same
 // places in shared memory, and so are its last reads and the next slot's first
-// writes: two barriers per slot.
+// writes: two barriers per slot.  FP32 lengths whose factors leave registers for
+// it load the next slot's points before the last half, which hides their latency
+// (us at 512 or 256 band pairs: 140^3 3590 -> 3310, 128^3 1405 -> 1321, 112^3
+// 465 -> 432, 84^3 111 -> 103).  Where the second factor is large, or a DFT of 9 or 15
+// points leaves nothing, the compiler spills and it costs 1 to 4 % (126^3 1371
+// -> 1421, 132^3 1429 -> 1448, 144^3 1698 -> 1745, 120^3 537 -> 541), and so in
+// FP64 (140^3 7510 -> 7730): these load at the start of their slot.
+template <typename T, int N> __host__ __device__ constexpr bool load_ahead() {
+  return sizeof(T) == 4 &&
+         (fac(N).r2 <= 8 ||
+          (fac(N).r1 >= 14 && fac(N).r1 % 3 != 0 && fac(N).r1 % 2 == 0 && fac(N).r2 % 2 == 0));
+}
+
 template <typename T, int N>
 __global__ void __launch_bounds__((lines<T, N>()) * fac(N).r1, (min_ctas<T, N, KXV>()))
 xv(Args a) {
@@ -552,15 +564,28 @@ xv(Args a) {
   const size_t ts = (size_t)g.ncol * nl;
   const int per = (a.nslots + gridDim.y - 1) / gridDim.y;
   const int e = min(a.nslots, (int)(blockIdx.y + 1) * per);
-  __syncthreads();
-  for (int slot = blockIdx.y * per; slot < e; ++slot) {
-    C* tile = (C*)a.tile + slot * ts + line;
-    C v[R1];
-    if (load) {
+  constexpr bool kAhead = load_ahead<T, N>();
+  C v[R1], next[kAhead ? R1 : 1];
+  auto fetch = [&](int slot, C (&x)[R1]) {
+    const C* in = (const C*)a.tile + slot * ts + line;
 #pragma unroll
-      for (int q = 0; q < R1; ++q) {
-        v[q] = cmk<C>(0, 0);
-        if (Keep<N>::q(q) && off[q] >= 0) v[q] = tile[off[q]];
+    for (int q = 0; q < R1; ++q) {
+      x[q] = cmk<C>(0, 0);
+      if (Keep<N>::q(q) && off[q] >= 0) x[q] = in[off[q]];
+    }
+  };
+  int slot = blockIdx.y * per;
+  if constexpr (kAhead)
+    if (load && slot < e) fetch(slot, next);
+  __syncthreads();
+  for (; slot < e; ++slot) {
+    C* tile = (C*)a.tile + slot * ts + line;
+    if (load) {
+      if constexpr (kAhead) {
+#pragma unroll
+        for (int q = 0; q < R1; ++q) v[q] = next[q];
+      } else {
+        fetch(slot, v);
       }
       first_half<N, +1>(v, item, tw, sm + item * kLines + lane, R2 * kLines);
     }
@@ -577,6 +602,8 @@ xv(Args a) {
       }
       first_half_rev<N, -1>(u, item, tw, sm + item * R2 * kLines + lane, kLines);
     }
+    if constexpr (kAhead)
+      if (load && slot + 1 < e) fetch(slot + 1, next);
     __syncthreads();
     if (load) {
 #pragma unroll
