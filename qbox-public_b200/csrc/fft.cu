@@ -1436,16 +1436,22 @@ void vb_forward_real3(Context& ctx, const double* f, const double* w, double* co
 }
 
 // out0 = add + back(a) and, with b, out1 = out0 + back(b): the sums over the
-// grid that follow a transform, in its last pass where the line passes run
+// grid that follow a transform, in its last pass where the line passes run.
+// Without b, out0 is not add and d_exc keeps its contents (the LDA's energy
+// density, which the stress reads later); with b, d_exc is scratch.
 void vb_backward_add(Context& ctx, const double* a, const double* b, const double* add,
                      double* out0, double* out1) {
   if (ctx.grid_zfast) return fields_backward(ctx, a, b, out0, out1, add, b != nullptr);
   const size_t N = ctx.N();
-  if (b) vb_backward_pair(ctx, a, b, (double*)ctx.d_exc, out1);
-  else vb_backward(ctx, a, ctx.d_exc);
+  if (!b) {
+    vb_backward(ctx, a, out0);
+    k_add<<<nblk(N), 256, 0, ctx.stream>>>(add, out0, N, out0);
+    QBX_LAUNCHED(ctx);
+    return;
+  }
+  vb_backward_pair(ctx, a, b, ctx.d_exc, out1);
   k_add<<<nblk(N), 256, 0, ctx.stream>>>(add, ctx.d_exc, N, out0);
   QBX_LAUNCHED(ctx);
-  if (!b) return;
   k_add<<<nblk(N), 256, 0, ctx.stream>>>(out0, out1, N, out1);
   QBX_LAUNCHED(ctx);
 }

@@ -603,7 +603,8 @@ void vb_forward_real_pair(Context& ctx, const double* f0, const double* f1, cons
 // three real fields f, f + N, f + 2 N from and (times w) to their coefficients
 void vb_backward3(Context& ctx, double* const c[3], double* f);
 void vb_forward_real3(Context& ctx, const double* f, const double* w, double* const c[3]);
-// out0 = add + back(a); with b also out1 = out0 + back(b) (d_exc is scratch)
+// out0 = add + back(a); with b also out1 = out0 + back(b) (d_exc is scratch then;
+// without b it keeps its contents, and out0 is not add)
 void vb_backward_add(Context& ctx, const double* a, const double* b, const double* add,
                      double* out0, double* out1);
 // whether the grids can be kept z fastest, and their conversion from and to
