@@ -840,6 +840,19 @@ void launch_identity_axpy(Context& ctx, double* t, const double* q, int n, doubl
   QBX_LAUNCHED(ctx);
 }
 
+__global__ void k_symmetrize_lower(double* q, int n) {
+  const size_t nn = (size_t)n * n;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nn;
+       i += (size_t)gridDim.x * blockDim.x) {
+    const int r = (int)(i % n), c = (int)(i / n);
+    if (r < c) q[i] = q[c + (size_t)r * n];
+  }
+}
+void launch_symmetrize_lower(Context& ctx, double* q, int n) {
+  k_symmetrize_lower<<<blocks_for((size_t)n * n), kThreads, 0, ctx.stream>>>(q, n);
+  QBX_LAUNCHED(ctx);
+}
+
 __global__ void k_avg(double* x, const double* t, size_t n) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x)

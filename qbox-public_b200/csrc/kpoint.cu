@@ -202,10 +202,21 @@ void ensure_zwork(Context& ctx) {
 void overlap_cholesky_k(Context& ctx, const double* c, int ngw, int status) {
   const int n = ctx.nst;
   double* L = znn(ctx, 0);
-  // the whole product: cuBLAS's herk does not split the long contraction
-  // (n = 128, 24 k rows: 0.84 ms against 0.13)
-  QBX_BLAS(cublasZgemm(ctx.blas, CUBLAS_OP_C, CUBLAS_OP_N, n, n, ngw, &kOne, zc(c), ngw, zc(c),
-                       ngw, &kZero, zc(L), n));
+  // The lower triangle by products of 256 columns with the rows from their diagonal
+  // block down, up to 1024 bands: cuBLAS's herk does not split the long contraction
+  // (ms of herk, whole product, these: n = 128, 24 k rows 0.85, 0.11, 0.11; n = 512,
+  // 6 k 0.41, 0.37, 0.30; n = 1024, 24 k 4.04, 5.59, 3.62; n = 2048, 24 k 12.8, 22.0,
+  // 12.9)
+  if (n > 1024) {
+    const double one = 1.0, zero = 0.0;
+    QBX_BLAS(cublasZherk(ctx.blas, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_C, n, ngw, &one, zc(c), ngw,
+                         &zero, zc(L), n));
+  }
+  for (int j = 0; n <= 1024 && j < n; j += 256) {
+    const cuDoubleComplex* cj = zc(c) + (size_t)j * ngw;
+    QBX_BLAS(cublasZgemm(ctx.blas, CUBLAS_OP_C, CUBLAS_OP_N, n - j, std::min(256, n - j), ngw, &kOne,
+                         cj, ngw, cj, ngw, &kZero, zc(L) + (size_t)j * n + j, n));
+  }
   QBX_SOLVER(cusolverDnZpotrf(ctx.solver, CUBLAS_FILL_MODE_LOWER, n, zc(L), n, zc(ctx.d_zwork),
                               ctx.zwork_len, ctx.d_status + status));
 }

@@ -662,6 +662,7 @@ void nonlocal_only(Context& ctx, bool hpsi, double* out);
 void diag(Context& ctx, bool eigvec, double* w);
 void launch_identity_axpy(Context& ctx, double* t, const double* q, int n,
                           double alpha);       // t = I + alpha*q
+void launch_symmetrize_lower(Context& ctx, double* q, int n);
 void launch_avg_transpose(Context& ctx, double* x, const double* t, int n);
 void launch_frob2(Context& ctx, const double* q, int n);   // SLOT_FROB = ||q||_F^2
 void launch_sumsq(Context& ctx, const double* x, size_t len, int slot);   // sum of x_i^2

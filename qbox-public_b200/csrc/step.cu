@@ -20,6 +20,47 @@ namespace qbx {
 
 static bool mixed(const Context& ctx) { return ctx.precision == MIXED; }
 
+// S = 2 c^T c for c K x n, the lower triangle.  cuBLAS's syrk forms half the tiles,
+// but does not split a long contraction over CTAs, and its time is a staircase in
+// n; dgemm splits, but forms the tiles above the diagonal too.  So: the whole
+// product where it is small, then products of 256 columns with the rows from their
+// diagonal block down, and syrk where those no longer win: more than 1536 columns,
+// or a contraction short against n.  ms of syrk, whole product, blocks:
+//   n =  128, K = 48000:  0.54,  0.065,   -      n = 1024, K = 12000:  0.86,  0.82,  0.51
+//   n =  432, K = 12000:  0.23,  0.155, 0.138    n = 1024, K = 145838: 10.6,  8.8,   5.7
+//   n =  512, K = 3000:   0.067, 0.072, 0.066    n = 1300, K = 12000:  0.86,  1.30,  0.83
+//   n =  768, K = 12000:  0.34,  0.44,  0.32     n = 2048, K = 48000:  6.7,  11.2,   6.8
+//   n =  768, K = 3000:   0.094, 0.12,  0.11     n = 3072, K = 48000: 13.5,  24.9,  14.9
+static void overlap_product(Context& ctx, const double* c, int K, int n, double* S) {
+  const double two = 2.0, zero = 0.0;
+  if (n > 1536 || (n > 480 && K < 8 * n)) {
+    QBX_BLAS(cublasDsyrk(ctx.blas, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T, n, K, &two, c, K, &zero,
+                         S, n));
+    return;
+  }
+  const int width = n <= 480 ? n : 256;
+  for (int j = 0; j < n; j += width)
+    QBX_BLAS(cublasDgemm(ctx.blas, CUBLAS_OP_T, CUBLAS_OP_N, n - j, std::min(width, n - j), K, &two,
+                         c + (size_t)j * K, K, c + (size_t)j * K, K, &zero,
+                         S + (size_t)j * n + j, n));
+}
+
+// C = alpha x^T x + beta C, all of it, x n x n: the whole product or syrk, whose time is
+// a staircase in n, and a kernel that completes it (ms of the whole product and of
+// syrk alone: n = 512 0.021 and 0.021, 640 0.035 and 0.028, 768 0.042 and 0.032, 900
+// 0.065 and 0.075, 1024 0.077 and 0.086, 1100 0.103 and 0.091, 2048 0.56 and 0.30)
+static void square_product(Context& ctx, int n, double alpha, const double* x, double beta,
+                           double* C) {
+  if (n <= 512 || (n > 768 && n <= 1024)) {
+    QBX_BLAS(cublasDgemm(ctx.blas, CUBLAS_OP_T, CUBLAS_OP_N, n, n, n, &alpha, x, n, x, n, &beta, C,
+                         n));
+    return;
+  }
+  QBX_BLAS(cublasDsyrk(ctx.blas, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T, n, n, &alpha, x, n, &beta, C,
+                       n));
+  launch_symmetrize_lower(ctx, C, n);
+}
+
 // S = 2 C^T C - c0 c0^T, lower triangle; overlap_cholesky: then S = L L^T in place.  In the
 // mixed path the product uses the BF16 split of c in slot `split` and the
 // diagonal is recomputed exactly in FP64.  The factorisation's info code
@@ -36,11 +77,7 @@ static void overlap(Context& ctx, const double* c, double* S, int split, bool di
     if (diag_from_split) overlap_diag_from_split(ctx, c, K, n, ctx.ldp, S);
     else overlap_diag_f64(ctx, c, K, n, S);
   } else {
-    // the whole product: cuBLAS's syrk forms half the tiles but does not split
-    // the long contraction (n = 128, K = 48 000: 0.25 ms against 0.04; n = 1024,
-    // K = 145 838: 10.6 against 8.8)
-    QBX_BLAS(cublasDgemm(ctx.blas, CUBLAS_OP_T, CUBLAS_OP_N, n, n, K, &two, c, K, c, K, &zero, S,
-                         n));
+    overlap_product(ctx, c, K, n, S);
     launch_rank1_fix(ctx, S, n, c, K, c, K, n, n, -1.0, true);
   }
 }
@@ -87,9 +124,8 @@ void gram(Context& ctx, bool split_overlap) {
 // q = I - x^T x (full matrix) and SLOT_FROB = ||q||_F^2
 static void polar_q(Context& ctx, const double* x, double* q) {
   const int n = ctx.nst;
-  const double one = 1.0, mone = -1.0;
   launch_identity_axpy(ctx, q, q, n, 0.0);   // q = I
-  QBX_BLAS(cublasDgemm(ctx.blas, CUBLAS_OP_T, CUBLAS_OP_N, n, n, n, &mone, x, n, x, n, &one, q, n));
+  square_product(ctx, n, -1.0, x, 1.0, q);
   launch_frob2(ctx, q, n);
 }
 
@@ -226,8 +262,7 @@ static void polar_higham_chol(Context& ctx, double* x, const double* q, double* 
   QBX_SOLVER(cusolverDnDpotrf(ctx.solver, CUBLAS_FILL_MODE_LOWER, n, qt, n, ctx.d_solver_work,
                               ctx.solver_lwork, ctx.d_status + ST_INFO_POLAR));
   lower_inverse(ctx, qt, n, t, xp);              // t = L^-1 (xp is free until the next product)
-  QBX_BLAS(cublasDgemm(ctx.blas, CUBLAS_OP_T, CUBLAS_OP_N, n, n, n, &one, t, n, t, n, &zero, xp,
-                       n));                      // S^-1 = W^T W
+  square_product(ctx, n, 1.0, t, 0.0, xp);   // S^-1 = W^T W
   launch_identity_axpy(ctx, qt, xp, n, 1.0);    // I + S^-1
   QBX_BLAS(cublasDgemm(ctx.blas, CUBLAS_OP_N, CUBLAS_OP_N, n, n, n, &half, x, n, qt, n, &zero, xp,
                        n));

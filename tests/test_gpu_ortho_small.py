@@ -19,9 +19,9 @@ pytestmark = pytest.mark.gpu
 BANDS = [1, 7, 15, 16, 17, 40, 97, 127, 128]
 
 
-def _ctx(bands, precision, small, xc="LDA"):
+def _ctx(bands, precision, small, xc="LDA", edges=(11.0, 10.0, 12.5)):
     pos = systems.diamond_supercell(10.26, 1, 0.03, 4)[:5]
-    s = systems.System("box", np.diag([11.0, 10.0, 12.5]), [systems.SI], [(0, p) for p in pos],
+    s = systems.System("box", np.diag(edges), [systems.SI], [(0, p) for p in pos],
                        20.0, bands, xc, 13)
     os.environ["QBX_ORTHO_SMALL"] = small
     try:
@@ -92,4 +92,41 @@ def test_lower_inverse_with_smaller_last_blocks(n):
     got, _ = ctx.lower_inverse(bad)
     np.testing.assert_allclose(got @ l, np.eye(n), rtol=0, atol=64 * n * np.finfo(float).eps)
     assert np.all(got[np.triu_indices(n, 1)] == 0.0)
+    ctx.close()
+
+
+@pytest.mark.parametrize("n,edges", [(130, (11.0, 10.0, 12.5)), (520, (15.0, 14.0, 15.0)),
+                                     (1024, (11.0, 10.0, 12.5)), (1025, (11.0, 10.0, 12.5))])
+def test_overlap_and_polar_products(n, edges):
+    """The overlap as one product (130 bands), by blocks of columns of which the
+    last is smaller (520) and as a triangle (1024: a contraction short against
+    the bands), and the polar iteration's products on both sides of their lines:
+    C orthonormal to n eps times the overlap's condition (10) after gram, and
+    polar's factor that of the SVD to n eps times the matrix's condition (6)."""
+    ctx = _ctx(n, capi.FP64, "1", edges=edges)
+    c = ctx.get_coeffs()
+    s = 2 * (c.conj() @ c.T).real - np.outer(c[:, 0].real, c[:, 0].real)
+    tol = 10 * n * np.finfo(float).eps
+    np.testing.assert_allclose(s, np.eye(n), rtol=0, atol=tol)
+    rng = np.random.default_rng(n)
+    q, _ = np.linalg.qr(rng.standard_normal((n, n)))
+    w, _ = np.linalg.qr(rng.standard_normal((n, n)))
+    x = q @ np.diag(np.linspace(0.4, 2.5, n)) @ w
+    for precision in (capi.FP64, capi.MIXED):
+        if precision == capi.MIXED:
+            ctx.close()
+            ctx = _ctx(n, precision, "1", edges=edges)
+        f, _ = ctx.polar(x, 1e-6, 20, False)
+        np.testing.assert_allclose(f, q @ w, rtol=0, atol=tol)
+    ctx.close()
+
+
+@pytest.mark.parametrize("n", [255, 257, 513, 700])
+def test_complex_overlap_by_blocks(n):
+    pos = systems.diamond_supercell(10.26, 1, 0.03, 4)[:5]
+    s = systems.System("box", np.diag([11.0, 10.0, 12.5]), [systems.SI], [(0, p) for p in pos],
+                       20.0, n, "LDA", 13).with_kpoints([((0.25, 0.1, 0.3), 1.0)])
+    ctx = capi.from_system(s, precision=capi.FP64)
+    c = ctx.get_kpoint_coeffs(0)
+    np.testing.assert_allclose(c.conj() @ c.T, np.eye(n), rtol=0, atol=10 * n * np.finfo(float).eps)
     ctx.close()
