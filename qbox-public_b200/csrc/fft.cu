@@ -772,16 +772,18 @@ void grid_from_caller(Context& ctx, const double* f, double* out) {
 }
 
 // With k points the grids are z fastest only if every k point's sphere runs
-// through the line passes; the density and potential that the context holds
-// move to the new order.
+// through the line passes; every field that the context holds moves to the new
+// order (a stress without a new step combines them point by point).
 void kpoints_grid_order(Context& ctx) {
   bool z = grid_zfast_possible(ctx);
   for (const KPointSet& kp : ctx.kpts) z = z && pencil_ok(ctx, kp.dks, false);
   if (z == ctx.grid_zfast) return;
-  for (double* f : {ctx.d_rhor, ctx.d_vr}) {
+  const size_t N = ctx.N();
+  for (double* f : {ctx.d_rhor, ctx.d_vr, ctx.d_vxc, ctx.d_exc, ctx.d_vx2, ctx.d_grad,
+                    ctx.d_grad + N, ctx.d_grad + 2 * N}) {
     if (z) grid_from_caller(ctx, f, (double*)ctx.d_grid);
     else grid_to_caller(ctx, f, (double*)ctx.d_grid);
-    QBX_CUDA(cudaMemcpyAsync(f, ctx.d_grid, ctx.N() * sizeof(double), cudaMemcpyDeviceToDevice,
+    QBX_CUDA(cudaMemcpyAsync(f, ctx.d_grid, N * sizeof(double), cudaMemcpyDeviceToDevice,
                              ctx.stream));
   }
   ctx.grid_zfast = z;

@@ -66,3 +66,40 @@ def test_stress_parts(route, xc, monkeypatch):
         for k in a:
             np.testing.assert_allclose(b[k], a[k], rtol=0, atol=1e-12 * max(1e-3, np.abs(a[k]).max()),
                                        err_msg=k)
+
+
+def _after_k_points(s, monkeypatch, env, k):
+    """The stress at Gamma from the fields of a step at k points, and the
+    density and V(r) before and after the return to Gamma."""
+    ctx = _ctx(s, monkeypatch, env)
+    ctx.scf_step()
+    sk = s.with_kpoints([(k, 1.0)])
+    ctx.set_kpoints([k], [1.0])
+    reach = np.abs(ctx.kpoint_miller(0)).max(0)
+    ctx.set_kpoint_coeffs(0, sk.kcoefficients(0, sk.kmiller(0)))
+    ctx.gram()
+    ctx.scf_step()
+    before = ctx.density(), ctx.vr()
+    ctx.set_kpoints([], [])
+    after = ctx.density(), ctx.vr()
+    parts = ctx.stress()[1]
+    ctx.close()
+    return reach, before, after, parts
+
+
+@pytest.mark.parametrize("xc", ["LDA", "PBE"])
+def test_fields_follow_the_order_of_the_grids(xc, monkeypatch):
+    """A k point whose sphere reaches beyond the line kernels' points takes the
+    grids to x fastest and the return to Gamma takes them back: every field
+    moves with them (FP64, as above)."""
+    s = _cell(xc=xc)
+    k = (2.0, 0.0, 0.0)
+    _, _, grid, _ = capi.host_basis(s.cell, s.ecut)
+    reach, before, after, parts = _after_k_points(s, monkeypatch, {}, k)
+    assert reach[0] > (grid[0] - 1) // 4            # not a line kernel's sphere
+    _, _, _, want = _after_k_points(s, monkeypatch, ROUTES[0], k)
+    for a, b in zip(before, after):
+        np.testing.assert_array_equal(a, b)
+    for q in want:
+        np.testing.assert_allclose(parts[q], want[q], rtol=0,
+                                   atol=1e-12 * max(1e-3, np.abs(want[q]).max()), err_msg=q)
