@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <complex>
 #include <cstdio>
+#include <type_traits>
 #include <vector>
 
 #include "fft_pencil.cuh"
@@ -714,6 +715,15 @@ k_zfft_fwd_k(const double2* __restrict__ zbuf, int ngw, int band0, DeviceSticks 
 
 // ------------------------------------------------------- line-pass FFTs
 // (fft_pencil.cuh) The grids of the plane-free passes: z fastest.
+// a grid value as the passes read it: FP64, or the value rounded to FP32 and the
+// rest (none where the rounded value is not finite)
+template <typename B> __device__ __forceinline__ B grid_value(double x);
+template <> __device__ __forceinline__ double grid_value<double>(double x) { return x; }
+template <> __device__ __forceinline__ float2 grid_value<float2>(double x) {
+  const float hi = (float)x;
+  return make_float2(hi, isfinite(hi) ? (float)(x - (double)hi) : 0.f);
+}
+
 // x-fastest grid <-> [x][y][z], 32 x 32 tiles of (x, z) at each y
 template <typename A, typename B, bool ADD>
 __global__ void __launch_bounds__(256)
@@ -725,14 +735,15 @@ k_grid_to_zfast(const A* __restrict__ in, int n0, int n1, int n2, bool to_zfast,
   for (int i = b; i < 32; i += 8) {
     const int x = to_zfast ? x0 + a : x0 + i, z = to_zfast ? z0 + i : z0 + a;
     if (x < n0 && z < n2)
-      t[i][a] = (B)in[to_zfast ? ((size_t)z * n1 + y) * n0 + x : ((size_t)x * n1 + y) * n2 + z];
+      t[i][a] = grid_value<B>(in[to_zfast ? ((size_t)z * n1 + y) * n0 + x : ((size_t)x * n1 + y) * n2 + z]);
   }
   __syncthreads();
   for (int i = b; i < 32; i += 8) {
     const int x = to_zfast ? x0 + i : x0 + a, z = to_zfast ? z0 + a : z0 + i;
     if (x < n0 && z < n2) {
       B* o = out + (to_zfast ? ((size_t)x * n1 + y) * n2 + z : ((size_t)z * n1 + y) * n0 + x);
-      *o = ADD ? *o + t[a][i] : t[a][i];
+      if constexpr (ADD) *o += t[a][i];
+      else *o = t[a][i];
     }
   }
 }
@@ -740,10 +751,10 @@ k_grid_to_zfast(const A* __restrict__ in, int n0, int n1, int n2, bool to_zfast,
 static int nblk(size_t n);
 static bool pencil_ok(const Context& ctx, const DeviceSticks& g, bool fp32);
 
-__global__ void k_to_float(const double* __restrict__ x, size_t n, float* __restrict__ y) {
+__global__ void k_to_floats(const double* __restrict__ x, size_t n, float2* __restrict__ y) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x)
-    y[i] = (float)x[i];
+    y[i] = grid_value<float2>(x[i]);
 }
 
 // The context's real-space grids (density, potentials, gradients) are kept z
@@ -901,12 +912,10 @@ static void pencil_pass(Context& ctx, const DeviceSticks& g, bool complex_basis,
   a.c = (const double2*)c;
   a.hc = (double2*)hc;
   a.g2 = g2;
-  // FP32: the gain of the rounded roots taken out (as 1 in FP64), the weights
-  // in units of 1/Omega so that whole occupations are exact
+  // FP32: the gain of the rounded roots taken out (as 1 in FP64)
   const double gain = sizeof(T) == 4 ? g.gain32 : 1.0;
   a.scale = 1.0 / ((double)N * gain);
-  a.wunit = sizeof(T) == 4 ? 1.0 / ctx.wb.omega : 1.0;
-  a.wout = a.wunit / gain;
+  a.wout = 1.0 / gain;
   a.ngw = ngw;
   a.nst = ctx.nst;
   a.w = w;
@@ -915,15 +924,16 @@ static void pencil_pass(Context& ctx, const DeviceSticks& g, bool complex_basis,
   // so (grid_zfast), else transposed through d_grid
   const bool zfast = ctx.grid_zfast;
   a.rho = zfast ? rho : (double*)ctx.d_grid;
-  T* vt = (T*)((double*)ctx.d_grid + N);
+  using V = std::conditional_t<sizeof(T) == 4, float2, double>;
+  V* vt = (V*)((double*)ctx.d_grid + N);
   a.v = vt;
   a.stream = ctx.stream;
   if (op == OP_VPSI) {
     if (zfast && sizeof(T) == 8) {
       a.v = v;
     } else {
-      if (zfast) k_to_float<<<nblk(N), 256, 0, ctx.stream>>>(v, N, (float*)vt);
-      else k_grid_to_zfast<double, T, false><<<tg, 256, 0, ctx.stream>>>(v, g.n0, g.n1, g.n2, true,
+      if (zfast) k_to_floats<<<nblk(N), 256, 0, ctx.stream>>>(v, N, (float2*)vt);
+      else k_grid_to_zfast<double, V, false><<<tg, 256, 0, ctx.stream>>>(v, g.n0, g.n1, g.n2, true,
                                                                         vt);
       QBX_LAUNCHED(ctx);
     }
@@ -945,8 +955,7 @@ static void pencil_pass(Context& ctx, const DeviceSticks& g, bool complex_basis,
                   : (void*)((C*)ctx.d_zfast + batch * (sb / sizeof(C)));
   };
   // CTAs per set of lines: enough for several per SM.  A CTA of the y passes
-  // takes up to 4 slots, one of the x passes up to 16 (the density sums that
-  // many slots in the context's precision before the FP64 sum)
+  // takes up to 4 slots, one of the x passes up to 16
   auto chunks = [&](int ns, int cta, int most) {
     return std::min(ns, std::max((ns + most - 1) / most, (1184 + cta - 1) / cta));
   };

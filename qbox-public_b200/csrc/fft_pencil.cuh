@@ -82,6 +82,15 @@ template <typename T, int N> __host__ __device__ constexpr int lines() {
   const int per = 2 * (int)sizeof(T) * (N + 2 * fac(N).r1 + 2);
   return 16 * per + 2 * (int)sizeof(T) * N <= 48 * 1024 ? 16 : 8;
 }
+// Of V(r) in FP32, two floats a point, xv holds in shared memory both (unless its
+// first DFT is of 14 points), or the second, or the second of the later points:
+// what fits in 48 KB.  lows: the second floats of a thread in registers.
+template <int N> __host__ __device__ constexpr bool v_shared() {
+  return fac(N).r1 != 14 && lines<float, N>() * (8 + 8) * N + 8 * N <= 48 * 1024;
+}
+template <int N> __host__ __device__ constexpr int v_lows() {
+  return lines<float, N>() * (8 + 4) * N + 8 * N <= 48 * 1024 ? 0 : fac(N).r2 / 2;
+}
 
 // CTAs per SM that the register file should hold.  The R1-point DFT sets what
 // a thread needs: with 14 points and more the y and x kernels want 72 registers
@@ -113,12 +122,12 @@ struct Args {
   void* tile = nullptr;
   int nslots = 0;
   int chunks = 1;                // CTAs that share the slots of one set of lines
-  const void* v = nullptr;       // V(r), [x][y][z]
+  const void* v = nullptr;       // V(r), [x][y][z]; FP32 passes: float2, the value rounded
+                                 // to FP32 and the rest
   double* rho = nullptr;         // density, [x][y][z]
   const double* w = nullptr;     // weights, two per slot (band n at w[n])
   int nw = 0;                    // weights in all; beyond: zero
-  double wunit = 1;              // the sums take the weights in this unit ...
-  double wout = 1;               // ... and are added to rho times this, in FP64
+  double wout = 1;               // the sums are added to rho times this
   bool rho_set = false;          // store the density instead of adding (chunks == 1)
   // real fields on a whole grid (the density basis, G* passes): two coefficient
   // arrays and two fields per slot, the second of each may be null
@@ -447,7 +456,10 @@ yf(Args a) {
 // Lines (y, z) flattened, from the occupied columns of the tile.  A CTA keeps
 // its lines over all slots of its chunk, so the density of a point stays in
 // a register until the chunk ends, and V(r) is read once.  The next slot's
-// loads are in flight over the second half.
+// loads are in flight over the second half.  The density's weights, products and
+// sums are FP64 in both precisions; with FP32 ones and these xd<float> takes (us) 72
+// and 73 at 84^3 (64 band pairs), 478 and 511 at 112^3 (216), 2140 and 2150 at 140^3
+// (512).
 template <int N>
 __device__ __forceinline__ void x_columns(const DeviceSticks& g, int item, int nl,
                                           int (&off)[fac(N).r1]) {
@@ -475,7 +487,7 @@ xd(Args a) {
   load_tw<C, N>(tw, a.tw[0]);
   int off[R1];
   if (item < R2) x_columns<N>(g, item, nl, off);
-  T acc[R2];
+  double acc[R2];
 #pragma unroll
   for (int m = 0; m < R2; ++m) acc[m] = 0;
   const size_t ts = (size_t)g.ncol * nl;
@@ -500,8 +512,8 @@ xd(Args a) {
       if (slot + 1 < e) fetch(slot + 1);   // in flight over the second half
     }
     const int n1 = 2 * (a.first + slot);
-    const T w1 = (T)(n1 < a.nw ? a.w[n1] / a.wunit : 0.0);
-    const T w2 = (T)(n1 + 1 < a.nw ? a.w[n1 + 1] / a.wunit : 0.0);
+    const double w1 = n1 < a.nw ? a.w[n1] : 0.0;
+    const double w2 = n1 + 1 < a.nw ? a.w[n1 + 1] : 0.0;
     __syncthreads();
     if (on) {
       C u[R2];
@@ -509,7 +521,10 @@ xd(Args a) {
       for (int j = 0; j < R2; ++j) u[j] = sm[(item * R2 + j) * kLines + lane];
       lane::dft_reg<R2, +1>(u);
 #pragma unroll
-      for (int m = 0; m < R2; ++m) acc[m] += w1 * u[m].x * u[m].x + w2 * u[m].y * u[m].y;
+      for (int m = 0; m < R2; ++m) {
+        const double p = u[m].x, q = u[m].y;
+        acc[m] = fma(w1 * p, p, fma(w2 * q, q, acc[m]));
+      }
     }
   }
   if (on) {
@@ -517,7 +532,7 @@ xd(Args a) {
 #pragma unroll
     for (int m = 0; m < R2; ++m) {
       double* p = rho + (size_t)m * R1 * nl;
-      const double x = a.wout * (double)acc[m];
+      const double x = a.wout * acc[m];
       if (gridDim.y > 1) atomicAdd(p, x);
       else *p = a.rho_set ? x : *p + x;
     }
@@ -527,26 +542,32 @@ xd(Args a) {
 // The tile in place: x transform to psi(r), times V(r), transform back.  A
 // thread's second-half reads and its writes of the way back are the same
 // places in shared memory, and so are its last reads and the next slot's first
-// writes: two barriers per slot.  FP32 lengths whose factors leave registers for
-// it load the next slot's points before the last half, which hides their latency
-// (us at 512 or 256 band pairs: 140^3 3590 -> 3310, 128^3 1405 -> 1321, 112^3
-// 465 -> 432, 84^3 111 -> 103).  Where the second factor is large, or a DFT of 9 or 15
-// points leaves nothing, the compiler spills and it costs 1 to 4 % (126^3 1371
-// -> 1421, 132^3 1429 -> 1448, 144^3 1698 -> 1745, 120^3 537 -> 541), and so in
-// FP64 (140^3 7510 -> 7730): these load at the start of their slot.
-template <typename T, int N> __host__ __device__ constexpr bool load_ahead() {
-  return sizeof(T) == 4 &&
-         (fac(N).r2 <= 8 ||
-          (fac(N).r1 >= 14 && fac(N).r1 % 3 != 0 && fac(N).r1 % 2 == 0 && fac(N).r2 % 2 == 0));
-}
-
+// writes: two barriers per slot.
+//   FP32: the product with V(r) is that with the FP64 value but for its own
+// rounding: V(r) is a float and the rest of it another, both in shared memory, two
+// packed instructions where V(r) rounded to FP32 in registers takes two scalar
+// ones (us of 64 slots of N x 96 x 96 points, V(r) rounded and whole: 64 82 and 85, 84
+// 132 and 132, 96 133 and 134, 128 207 and 214, 144 221 and 214).  With the 14-point
+// DFT, and where the room is short, only the rest is there (112 171 -> 185, both in
+// shared memory 190; 140 218 -> 236, both 245; 224 337 -> 362; all in registers spills:
+// 140 240, 224 380).
+//   FP32 also loads the next slot's points before the last half, which hides their
+// latency (without and with: 60 112 -> 102, 84 151 -> 140, 96 153 -> 142, 140 248 ->
+// 235, 192 335 -> 309, 240 427 -> 404; equal within 2 % at 126 and 144, and 82 -> 87 at
+// 56, 153 -> 157 at 90).  In FP64 (7510 -> 7730 us at 140^3, 512 band pairs) the compiler
+// spills, and the points are loaded at the start of their slot.
 template <typename T, int N>
 __global__ void __launch_bounds__((lines<T, N>()) * fac(N).r1, (min_ctas<T, N, KXV>()))
 xv(Args a) {
   using C = typename CT<T>::c;
   constexpr int R1 = fac(N).r1, R2 = fac(N).r2, kLines = lines<T, N>();
+  constexpr bool kFloat = sizeof(T) == 4, kAhead = kFloat, kBoth = kFloat && v_shared<N>();
+  constexpr int kLows = kFloat ? v_lows<N>() : 0, kRest = R2 - kLows;
   __shared__ C tw[N];
   __shared__ C sm[N * kLines];
+  // [k][j] as sm; an entry is its thread's own
+  __shared__ float2 vall[kBoth ? N * kLines : 1];
+  __shared__ float vrest[kFloat && !kBoth ? R1 * kRest * kLines : 1];
   const DeviceSticks& g = a.g;
   const int lane = threadIdx.x % kLines, item = threadIdx.x / kLines;
   const int line = blockIdx.x * kLines + lane;
@@ -555,16 +576,28 @@ xv(Args a) {
   load_tw<C, N>(tw, a.tw[0]);
   int off[R1];
   if (item < R2) x_columns<N>(g, item, nl, off);
-  T vr[R2];
+  T vr[kBoth ? 1 : R2], vlow[kLows ? kLows : 1];
   if (on) {
-    const T* v = (const T*)a.v + (size_t)item * nl + line;
+    const size_t p = (size_t)item * nl + line;
 #pragma unroll
-    for (int m = 0; m < R2; ++m) vr[m] = v[(size_t)m * R1 * nl];
+    for (int m = 0; m < R2; ++m) {
+      if constexpr (kFloat) {
+        const float2 v = ((const float2*)a.v)[p + (size_t)m * R1 * nl];
+        if constexpr (kBoth) {
+          vall[(item * R2 + m) * kLines + lane] = v;
+        } else {
+          vr[m] = v.x;
+          if (m < kLows) vlow[m < kLows ? m : 0] = v.y;
+          else vrest[(item * kRest + m - kLows) * kLines + lane] = v.y;
+        }
+      } else {
+        vr[m] = ((const double*)a.v)[p + (size_t)m * R1 * nl];
+      }
+    }
   }
   const size_t ts = (size_t)g.ncol * nl;
   const int per = (a.nslots + gridDim.y - 1) / gridDim.y;
   const int e = min(a.nslots, (int)(blockIdx.y + 1) * per);
-  constexpr bool kAhead = load_ahead<T, N>();
   C v[R1], next[kAhead ? R1 : 1];
   auto fetch = [&](int slot, C (&x)[R1]) {
     const C* in = (const C*)a.tile + slot * ts + line;
@@ -597,8 +630,16 @@ xv(Args a) {
       lane::dft_reg<R2, +1>(u);
 #pragma unroll
       for (int m = 0; m < R2; ++m) {
-        u[m].x *= vr[m];
-        u[m].y *= vr[m];
+        if constexpr (kFloat) {
+          float2 v;
+          if constexpr (kBoth) v = vall[(item * R2 + m) * kLines + lane];
+          else v = make_float2(vr[m], m < kLows ? vlow[m < kLows ? m : 0]
+                                      : vrest[(item * kRest + m - kLows) * kLines + lane]);
+          u[m] = reg::cfma(u[m], v.x, reg::cscale(u[m], v.y));
+        } else {
+          u[m].x *= vr[m];
+          u[m].y *= vr[m];
+        }
       }
       first_half_rev<N, -1>(u, item, tw, sm + item * R2 * kLines + lane, kLines);
     }

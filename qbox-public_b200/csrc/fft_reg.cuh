@@ -72,6 +72,15 @@ __device__ __forceinline__ float2 cfma(float2 a, float s, float2 b) {
       : "f"(a.x), "f"(a.y), "f"(s), "f"(b.x), "f"(b.y));
   return r;
 }
+// a s for a real s
+__device__ __forceinline__ float2 cscale(float2 a, float s) {
+  float2 r;
+  asm("{.reg .b64 p, q, u;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %4};\n\t"
+      "mul.rn.f32x2 u, p, q;\n\tmov.b64 {%0, %1}, u;}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(s));
+  return r;
+}
 template <typename C> __device__ __forceinline__ C cmul(C a, C b) {
   C r; r.x = a.x * b.x - a.y * b.y; r.y = a.x * b.y + a.y * b.x; return r;
 }

@@ -7,8 +7,8 @@ kept from the density pass against transforming twice (QBX_PSIR=0).
 FP64: the same sums in another order, 1e-12 of the largest value.  FP32: one
 rounding of 6e-8 per butterfly level on three axes, 2e-6 of the largest
 value; the charge, whose systematic part the passes take out, 1e-7 of the
-electrons (the FP32 sum of at most 16 bands and the FFT's rounding average
-out over the grid).
+electrons (the FFT's rounding averages out over the grid).  In FP32 too the
+density's weights, products and sums are FP64 and V(r) keeps its FP64 value.
 """
 import os
 
@@ -94,3 +94,90 @@ def test_kept_tiles_give_the_recomputed_step(precision, kpoints):
     np.testing.assert_allclose(ea, eb, rtol=1e-12)
     for a, b in zip(ca, cb):
         np.testing.assert_allclose(a, b, rtol=0, atol=1e-11)
+
+
+def _mixed_box(bands):
+    """64 x 32 x 64 points: the sums of a constant are exact in FP32, and a
+    CTA of the x passes takes 16 slots of 320 bands."""
+    return _cell(20.0, 9.75, 19.75, 20.0, bands)
+
+
+def _constant(ctx, values):
+    """Band n constant in r: its G = 0 coefficient alone."""
+    c = np.zeros((ctx.nst, ctx.ngw), complex)
+    g0 = int(np.flatnonzero(~ctx.miller().any(axis=1))[0])
+    c[:, g0] = values
+    ctx.set_coeffs(c)
+    return g0
+
+
+@pytest.mark.parametrize("fast", ["1", "0"])
+def test_mixed_density_sums_in_fp64(fast, tmp_path):
+    """Constant bands whose values FP32 holds: the density is sum_n f_n c_n^2 /
+    Omega times one factor (the gain that the passes take out), for fractional
+    occupations too.  A product, weight or sum of 16 slots in FP32 shows at
+    1e-8; FP64 leaves 320 roundings, 1e-13."""
+    bands = 320
+    os.environ["QBX_FAST_FFT"] = fast
+    try:
+        ctx = capi.from_system(_mixed_box(bands), precision=capi.MIXED, gram=False)
+    finally:
+        os.environ.pop("QBX_FAST_FFT")
+    assert tuple(ctx.grid) == (64, 32, 64)
+    rng = np.random.default_rng(4)
+    values = 1.0 + rng.integers(0, 1 << 12, bands) / (1 << 12)
+    # occupations come with a sample's <wavefunction>
+    path = str(tmp_path / "wf.xml")
+    ctx.write_wavefunction(path)
+    text = open(path).read()
+    a = text.index(">", text.index("<density_matrix")) + 1
+    b = text.index("</density_matrix>")
+    factor = []
+    for occ in (np.full(bands, 2.0), rng.uniform(0.1, 2.0, bands), rng.uniform(0.1, 2.0, bands)):
+        with open(path, "w") as f:
+            f.write(text[:a] + "\n" + "\n".join(repr(float(o)) for o in occ) + "\n" + text[b:])
+        ctx.read_wavefunction(path)
+        _constant(ctx, values)
+        ctx.update_density()
+        rho = ctx.density()
+        factor += [rho.min() / np.dot(occ, values ** 2), rho.max() / np.dot(occ, values ** 2)]
+    ctx.close()
+    np.testing.assert_allclose(factor, factor[0], rtol=1e-13)
+
+
+@pytest.mark.parametrize("fast", ["1", "0"])
+def test_mixed_product_with_the_fp64_potential(fast):
+    """A constant band times a constant V: FP32 rounds the product with the
+    FP64 value of V, which here is one unit off the product with V rounded to
+    FP32 first."""
+    os.environ["QBX_FAST_FFT"] = fast
+    try:
+        ctx = capi.from_system(_mixed_box(4), precision=capi.MIXED, gram=False)
+    finally:
+        os.environ.pop("QBX_FAST_FFT")
+    x = np.float32([1.9, 1.99, 1.75, 1.95]).astype(float)
+    g0 = _constant(ctx, x)
+    out = []
+    v = 1.0 + 0.98 * 2.0 ** -24
+    for pot in (1.0, v):
+        dc = np.zeros((ctx.nst, ctx.ngw), complex)
+        ctx.rs_mul_add(np.full(int(np.prod(ctx.grid)), pot), dc)
+        out.append(dc[:, g0].real.copy())
+    ctx.close()
+    want = (x * v).astype(np.float32).astype(float)
+    assert np.float32(v) == 1.0 and np.all(want > x)
+    np.testing.assert_allclose(out[1] / out[0], want / x, rtol=1e-12)
+
+
+def test_mixed_density_of_long_slot_chunks():
+    """320 bands, 16 slots a CTA, against FP64 point by point: the transforms'
+    rounding (17 butterfly levels of 6e-8 in each of 320 bands, independent),
+    2e-7 of the largest value."""
+    s = _mixed_box(320)
+    rho = []
+    for precision in (capi.FP64, capi.MIXED):
+        ctx = capi.from_system(s, precision=precision)
+        ctx.update_density()
+        rho.append(ctx.density())
+        ctx.close()
+    np.testing.assert_allclose(rho[1], rho[0], rtol=0, atol=2e-7 * np.abs(rho[0]).max())
