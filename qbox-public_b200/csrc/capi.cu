@@ -564,6 +564,7 @@ int qbx_set_cell(qbx_context* h, const double cell[9], double ecut, int nst, con
       c.d_vr32 = dalloc<float>(N);
       c.fast_fft = true;
       if (const char* e = std::getenv("QBX_FAST_FFT")) c.fast_fft = std::atoi(e) != 0;
+      c.wtile_mode = -1;   // room is looked for again with each cell
       if (const char* e = std::getenv("QBX_PSIR")) c.wtile_mode = std::atoi(e) != 0 ? 1 : 0;
     }
     c.grid_zfast = grid_zfast_possible(c);
