@@ -875,21 +875,28 @@ static bool pencil_ok(const Context& ctx, const DeviceSticks& g, bool fp32) {
 // The buffer that keeps every slot's tile (`need` bytes): allocated, outside
 // stream capture, when `keep` asks for it and the device has room; without
 // `keep` only a buffer that is there already.  Null: no such buffer, and the
-// tiles go through the stick buffer in batches.
+// tiles go through the stick buffer in batches.  Room is twice the buffer and 4 GB,
+// since a context works without it: as much again is left to the contexts that a
+// program makes after this one's first step.
 static void* tile_area(Context& ctx, size_t need, bool keep) {
   if (ctx.d_wtile && ctx.wtile_bytes >= need) return ctx.d_wtile;
   if (!keep || ctx.wtile_mode == 0 || ctx.capturing) return nullptr;
   size_t freeb = 0, total = 0;
   QBX_CUDA(cudaMemGetInfo(&freeb, &total));
-  if (freeb < need + ((size_t)4 << 30)) {
-    if (ctx.wtile_mode < 0) ctx.wtile_mode = 0;   // no room: transform twice from now on
-    return nullptr;
+  if (freeb >= 2 * need + ((size_t)4 << 30)) {
+    if (ctx.d_wtile) cudaFree(ctx.d_wtile);
+    ctx.d_wtile = nullptr;
+    const cudaError_t e = cudaMalloc(&ctx.d_wtile, need);
+    if (e == cudaSuccess) {
+      ctx.wtile_bytes = need;
+      return ctx.d_wtile;
+    }
+    ctx.d_wtile = nullptr;
+    if (e != cudaErrorMemoryAllocation) QBX_CUDA(e);
+    cudaGetLastError();   // taken by another context or process since
   }
-  if (ctx.d_wtile) cudaFree(ctx.d_wtile);
-  ctx.d_wtile = nullptr;
-  QBX_CUDA(cudaMalloc(&ctx.d_wtile, need));
-  ctx.wtile_bytes = need;
-  return ctx.d_wtile;
+  if (ctx.wtile_mode < 0) ctx.wtile_mode = 0;   // no room: transform twice for this cell
+  return nullptr;
 }
 
 // Slots first ... first + nslots of one wavefunction block (band pairs, or

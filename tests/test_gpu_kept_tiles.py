@@ -72,3 +72,24 @@ def test_room_is_looked_for_again_with_each_cell(precision):
     _load(ctx, s)
     assert _launches(ctx) == kept
     ctx.close()
+
+
+def test_as_much_room_is_left_as_the_tiles_take():
+    """256 bands of the 512-atom cell in FP64, 2.9 GB of tiles: kept where 12 GB are
+    free, not where 8 GB are, so that a context made next still finds its memory."""
+    s = systems.si512().band_sample(256)
+    ctx = capi.Context(0, capi.FP64)
+    _load(ctx, s)
+    _, _, grid, hkl = capi.host_basis(s.cell, s.ecut)
+    need = s.nbands // 2 * 16 * (2 * int(hkl[:, 0].max()) + 1) * grid[1] * grid[2]
+    assert 2 * need + 4 * GB < 12 * GB and need + 4 * GB < 8 * GB < 2 * need + 4 * GB
+    used = []
+    for left in (8 * GB, 12 * GB):
+        _load(ctx, s)
+        full = _Full(left)
+        try:
+            used.append(_launches(ctx))
+        finally:
+            full.release()
+    ctx.close()
+    assert used[0] > used[1]
