@@ -91,8 +91,8 @@ void free_cell(Context& c) {
   dfree(c.d_info);
   if (c.d_grid) { cudaFree(c.d_grid); c.d_grid = nullptr; }
   if (c.d_zbuf) { cudaFree(c.d_zbuf); c.d_zbuf = nullptr; }
+  c.zbuf_bytes = 0;
   if (c.d_zfast) { cudaFree(c.d_zfast); c.d_zfast = nullptr; }
-  dfree(c.d_vr32);
   c.have_cell = false;
 }
 
@@ -467,14 +467,8 @@ int qbx_set_precision(qbx_context* h, int precision) {
   return guarded(h, [&](Context& c) {
     QBX_REQUIRE(precision == QBX_FP64 || precision == QBX_MIXED, 1, "unknown precision");
     if (c.have_cell && precision != c.precision) {
-      // the stick buffer holds the precision's complex type
       c.precision = precision;
-      const size_t per_pair = (size_t)c.wb.n2 * c.wb.nvec *
-                              (precision == QBX_MIXED ? sizeof(float2) : sizeof(double2));
-      if (c.d_zbuf) cudaFree(c.d_zbuf);
-      c.d_zbuf = nullptr;
-      QBX_CUDA(cudaMalloc(&c.d_zbuf, per_pair * c.pair_batch));
-      c.zbuf_bytes = per_pair * c.pair_batch;
+      ensure_radix_buffer(c);
     }
     c.precision = precision;
     drop_graphs(c);
@@ -547,13 +541,11 @@ int qbx_set_cell(qbx_context* h, const double cell[9], double ecut, int nst, con
     c.d_scalars = dalloc<double>(kSlots + nst);
     QBX_CUDA(cudaMemset(c.d_scalars, 0, kSlots * sizeof(double)));
     upload_weights(c);
-    // staged FFT stick buffer: bounded to ~4 GB per batch of band pairs
+    // batch of the runtime-radix kernels, whose stick buffer is bounded to 4 GB
     const int npairs = (nst + 1) / 2;
     const size_t per_pair = (size_t)c.wb.n2 * c.wb.nvec *
                             (c.precision == QBX_MIXED ? sizeof(float2) : sizeof(double2));
     c.pair_batch = (int)std::max<size_t>(1, std::min<size_t>(npairs, ((size_t)4 << 30) / per_pair));
-    QBX_CUDA(cudaMalloc(&c.d_zbuf, per_pair * c.pair_batch));
-    c.zbuf_bytes = per_pair * c.pair_batch;
     // stick buffer of the line passes, in batches of band pairs
     {
       size_t mb = 256;
@@ -561,13 +553,13 @@ int qbx_set_cell(qbx_context* h, const double cell[9], double ecut, int nst, con
       const size_t pp64 = (size_t)c.wb.n2 * c.wb.nvec * sizeof(double2);
       c.zfast_bytes = std::max(mb << 20, pp64);
       QBX_CUDA(cudaMalloc(&c.d_zfast, c.zfast_bytes));
-      c.d_vr32 = dalloc<float>(N);
       c.fast_fft = true;
       if (const char* e = std::getenv("QBX_FAST_FFT")) c.fast_fft = std::atoi(e) != 0;
       c.wtile_mode = -1;   // room is looked for again with each cell
       if (const char* e = std::getenv("QBX_PSIR")) c.wtile_mode = std::atoi(e) != 0 ? 1 : 0;
     }
     c.grid_zfast = grid_zfast_possible(c);
+    ensure_radix_buffer(c);
     c.species.clear();
     c.tau.clear();
     QBX_CUDA(cudaDeviceSynchronize());   // memsets above ran on the legacy stream

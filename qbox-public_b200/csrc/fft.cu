@@ -766,6 +766,21 @@ bool grid_zfast_possible(const Context& ctx) {
          sizeof(double2) * (size_t)g.n2 * ((size_t)g.nvec + (size_t)g.ncol * g.n1);
 }
 
+// The runtime-radix kernels' stick buffer (up to 4 GB), for contexts whose
+// Gamma sphere or one of whose k points is not the line passes'; the precision
+// sets its size.
+void ensure_radix_buffer(Context& ctx) {
+  bool radix = !pencil_ok(ctx, ctx.dws, ctx.precision == MIXED);
+  for (const KPointSet& kp : ctx.kpts) radix = radix || !pencil_ok(ctx, kp.dks, false);
+  const size_t need = density_stick_bytes_per_pair(ctx) * ctx.pair_batch;
+  if (!radix || ctx.zbuf_bytes == need) return;
+  if (ctx.d_zbuf) cudaFree(ctx.d_zbuf);
+  ctx.d_zbuf = nullptr;
+  ctx.zbuf_bytes = 0;
+  QBX_CUDA(cudaMalloc(&ctx.d_zbuf, need));
+  ctx.zbuf_bytes = need;
+}
+
 // f as callers see it (x fastest), in `out`; and the opposite
 void grid_to_caller(Context& ctx, const double* f, double* out) {
   const DeviceSticks& g = ctx.dvs;
@@ -786,6 +801,7 @@ void grid_from_caller(Context& ctx, const double* f, double* out) {
 // through the line passes; every field that the context holds moves to the new
 // order (a stress without a new step combines them point by point).
 void kpoints_grid_order(Context& ctx) {
+  ensure_radix_buffer(ctx);
   bool z = grid_zfast_possible(ctx);
   for (const KPointSet& kp : ctx.kpts) z = z && pencil_ok(ctx, kp.dks, false);
   if (z == ctx.grid_zfast) return;

@@ -368,7 +368,7 @@ struct Context {
   double* d_vps = nullptr;      // ngv*nsp
   double* d_rhops_sp = nullptr; // ngv*nsp
   void* d_grid = nullptr;       // N complex (double2) scratch for vbasis FFTs
-  void* d_zbuf = nullptr;       // staged FFT stick buffer
+  void* d_zbuf = nullptr;       // stick buffer of the runtime-radix kernels, where they run
   size_t zbuf_bytes = 0;
   int pair_batch = 0;
   double* d_nn = nullptr;       // nst*nst matrices (4 of them)
@@ -457,7 +457,6 @@ struct Context {
   int ldp = 0;                  // padded leading dimension of the K-row splits
   float* c32 = nullptr;         // TF32 hi/lo split of C (tall updates)
   float* c32lo = nullptr;
-  float* d_vr32 = nullptr;      // FP32 copy of V(r) for the mixed H*psi pass
   void* d_zfast = nullptr;      // stick buffer of the specialised staged FFTs
   size_t zfast_bytes = 0;
   bool grid_zfast = false;      // the real-space grids are kept z fastest (fft.cu)
@@ -610,6 +609,8 @@ void vb_backward_add(Context& ctx, const double* a, const double* b, const doubl
 // whether the grids can be kept z fastest, and their conversion from and to
 // the callers' x-fastest order (device arrays)
 bool grid_zfast_possible(const Context& ctx);
+// d_zbuf, if some pass of this context runs the runtime-radix kernels
+void ensure_radix_buffer(Context& ctx);
 void kpoints_grid_order(Context& ctx);   // after the set of k points changed
 void grid_to_caller(Context& ctx, const double* f, double* out);
 void grid_from_caller(Context& ctx, const double* f, double* out);

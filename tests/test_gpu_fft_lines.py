@@ -181,3 +181,26 @@ def test_mixed_density_of_long_slot_chunks():
         rho.append(ctx.density())
         ctx.close()
     np.testing.assert_allclose(rho[1], rho[0], rtol=0, atol=2e-7 * np.abs(rho[0]).max())
+
+
+@pytest.mark.parametrize("fast", ["1", "0"])
+def test_precision_switch(fast):
+    """qbx_set_precision on either route and back: the buffers of the new
+    precision are there (the runtime-radix kernels' only where they run)."""
+    os.environ["QBX_FAST_FFT"] = fast
+    try:
+        ctx = capi.from_system(_cell(12.0, 7.5, 19.0, 20.0, 9), precision=capi.FP64)
+    finally:
+        os.environ.pop("QBX_FAST_FFT")
+    rho, h = [], []
+    for precision in (capi.FP64, capi.MIXED, capi.FP64):
+        ctx.set_precision(precision)
+        ctx.update_density()
+        ctx.update_vhxc()
+        ctx.energy(hpsi=True)
+        rho.append(ctx.density())
+        h.append(ctx.get_hpsi())
+    ctx.close()
+    for i, tol in ((1, 2e-6), (2, 1e-12)):
+        np.testing.assert_allclose(rho[i], rho[0], rtol=0, atol=tol * np.abs(rho[0]).max())
+        np.testing.assert_allclose(h[i], h[0], rtol=0, atol=tol * np.abs(h[0]).max())
