@@ -8,14 +8,15 @@
 #include <cstring>
 #include <fstream>
 #include <map>
+#include <memory>
 #include <sstream>
 #include <new>
 #include <stdexcept>
 #include <thread>
-#include <atomic>
 #include <tuple>
 
 #include "../../include/qbx.h"
+#include "host_add.h"
 #include "qbx_internal.h"
 
 struct qbx_context {
@@ -1403,13 +1404,15 @@ void upload_wf(qbx_context* h, const double* src, double* dst) {
 }
 
 // dst[i] += scale * src[i], src on the device (all of it written by work already
-// on c.stream), dst the caller's array.  1 MB pieces through pinned slots of the
-// context, each slot served by a thread that waits for its copy and adds it, so
-// that the copies run on while the additions, which the host's memory bounds,
-// are spread over the threads.  (Into a fresh vector and added by one thread,
-// 20 MB took 7 ms, most of it page faults and the addition.)
+// on c.stream), dst the caller's array, which keeps its values if a copy fails.
+// 1 MB pieces through pinned slots of the context, each slot served by a thread
+// that waits for its copy and adds it, so that the copies run on while the
+// additions, which the host's memory bounds, are spread over the threads.  (Into a
+// fresh vector and added by one thread, 20 MB took 7 ms, most of it page faults and
+// the addition.)  The old values are kept meanwhile, in a block that stays with
+// the context up to 64 MB.
 void add_to_caller(Context& c, const double* src, size_t n, double scale, double* dst) {
-  constexpr size_t kPiece = (size_t)1 << 17;
+  constexpr size_t kPiece = (size_t)1 << 17, kKeep = (size_t)8 << 20;
   const size_t pieces = (n + kPiece - 1) / kPiece;
   const size_t most = std::max(1u, std::thread::hardware_concurrency() / 2);
   const int nt = (int)std::min({pieces, (size_t)Context::kStageSlots, most});
@@ -1418,35 +1421,29 @@ void add_to_caller(Context& c, const double* src, size_t n, double scale, double
   for (int t = 0; t < nt; t++) {
     if (!c.ev_stage[t]) QBX_CUDA(cudaEventCreateWithFlags(&c.ev_stage[t], cudaEventDisableTiming));
   }
-  std::atomic<int> failed{0};
-  auto serve = [&](int t) {
-    if (cudaSetDevice(c.device) != cudaSuccess) failed = 1;
-    for (size_t i = t; i < pieces && !failed; i += nt) {
-      const size_t off = i * kPiece, m = std::min(kPiece, n - off);
-      double* buf = c.h_stage + t * kPiece;
-      if (cudaMemcpyAsync(buf, src + off, m * sizeof(double), cudaMemcpyDeviceToHost,
-                          c.stream) != cudaSuccess ||
-          cudaEventRecord(c.ev_stage[t], c.stream) != cudaSuccess ||
-          cudaEventSynchronize(c.ev_stage[t]) != cudaSuccess) {
-        failed = 1;
-        break;
-      }
-      double* d = dst + off;
-      for (size_t k = 0; k < m; k++) d[k] += scale * buf[k];
-    }
-  };
-  std::vector<std::thread> others;
-  int served = 1;                    // slots whose pieces someone serves
-  try {
-    for (; served < nt; served++) others.emplace_back(serve, served);
-  } catch (const std::exception&) {
-    // no thread to be had: this one serves the rest
+  std::unique_ptr<double[]> own;
+  if (n > kKeep) {
+    own.reset(new double[n]);
+  } else if (c.h_block_elems < n) {
+    c.h_block.reset();
+    c.h_block_elems = 0;
+    c.h_block.reset(new double[n]);
+    c.h_block_elems = n;
   }
-  serve(0);
-  for (int t = served; t < nt; t++) serve(t);
-  for (std::thread& t : others) t.join();
-  QBX_REQUIRE(!failed, 2, std::string("copy to the caller's array: ") +
-                              cudaGetErrorString(cudaGetLastError()));
+  const int code = add_all_or_nothing(
+      n, kPiece, nt, scale, own ? own.get() : c.h_block.get(), dst,
+      [&](int t, size_t first, size_t count, const double** x) -> int {
+        double* buf = c.h_stage + t * kPiece;
+        cudaError_t e = cudaSetDevice(c.device);
+        if (e == cudaSuccess)
+          e = cudaMemcpyAsync(buf, src + first, count * sizeof(double), cudaMemcpyDeviceToHost,
+                              c.stream);
+        if (e == cudaSuccess) e = cudaEventRecord(c.ev_stage[t], c.stream);
+        if (e == cudaSuccess) e = cudaEventSynchronize(c.ev_stage[t]);
+        *x = buf;
+        return (int)e;
+      });
+  if (code) QBX_CUDA((cudaError_t)code);
 }
 
 // a wavefunction block (internal order) added to the caller's (its order)

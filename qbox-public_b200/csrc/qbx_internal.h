@@ -15,6 +15,7 @@
 #include <complex>
 #include <iosfwd>
 #include <functional>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -516,9 +517,11 @@ struct Context {
   double last_energies[16] = {0};
   // pinned 1 MB pieces through which the class-level entry points add to the
   // caller's arrays, allocated on first use
-  static constexpr int kStageSlots = 6;
+  static constexpr int kStageSlots = 8;
   double* h_stage = nullptr;
   cudaEvent_t ev_stage[kStageSlots] = {nullptr};
+  std::unique_ptr<double[]> h_block;   // those arrays' old values meanwhile, up to 64 MB
+  size_t h_block_elems = 0;
   // k points off Gamma; when set, the electronic step runs on them instead
   // of the Gamma coefficients
   std::vector<KPointSet> kpts;
