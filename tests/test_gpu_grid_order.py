@@ -103,3 +103,82 @@ def test_fields_follow_the_order_of_the_grids(xc, monkeypatch):
     for q in want:
         np.testing.assert_allclose(parts[q], want[q], rtol=0,
                                    atol=1e-12 * max(1e-3, np.abs(want[q]).max()), err_msg=q)
+
+
+def _fields(ctx):
+    ctx.update_density()
+    ctx.update_vhxc()
+    e = ctx.energy(hpsi=True)
+    return ctx.density(), ctx.vr(), ctx.get_hpsi(), e
+
+
+@pytest.mark.parametrize("precision", [capi.FP64, capi.MIXED])
+@pytest.mark.parametrize("xc,edges", [("LDA", (12.0, 7.5, 19.0)), ("PBE", (12.0, 7.5, 19.0)),
+                                      ("PBE", (9.0, 16.5, 6.0))])
+@pytest.mark.parametrize("psir", ["0", "1"])
+def test_line_passes_on_x_fastest_grids(psir, xc, edges, precision, monkeypatch):
+    """The passes that transpose the density and V(r) against those that read and
+    write them in place, in one and in several batches of slots; at 30 x 56 x 22
+    the small buffer takes one slot of the density basis and the GGA's components go
+    through one transform at a time (FP64: the same arithmetic, 1e-12 of the largest
+    value; mixed: V(r) differs in its last bits, 2e-6)."""
+    s = _cell(edges=edges, bands=9, xc=xc)
+    out = []
+    for env in ({}, dict(ROUTES[1], QBX_PSIR=psir)):
+        ctx = _ctx(s, monkeypatch, env, precision)
+        f = _fields(ctx)
+        steps = [ctx.scf_step()["etotal"] for _ in range(2)]
+        out.append((f, steps))
+        ctx.close()
+    (fa, sa), (fb, sb) = out
+    tol = 1e-12 if precision == capi.FP64 else 2e-6
+    for a, b in zip(fa[:3], fb[:3]):
+        np.testing.assert_allclose(b, a, rtol=0, atol=tol * np.abs(a).max())
+    etol = 1e-11 if precision == capi.FP64 else 1e-7
+    for k in fa[3]:
+        if isinstance(fa[3][k], float):
+            assert abs(fa[3][k] - fb[3][k]) <= etol * max(1.0, abs(fa[3][k])), k
+    np.testing.assert_allclose(sb, sa, rtol=etol)
+
+
+@pytest.mark.parametrize("mb", [40, 100])
+@pytest.mark.parametrize("psir", ["0", "1"])
+@pytest.mark.parametrize("precision", [capi.FP64, capi.MIXED])
+def test_smaller_stick_buffers(precision, psir, mb, monkeypatch):
+    """140^3, 16 band pairs (FP64 30 MB a pair): buffers that take the slots in
+    several batches, no slot of the density basis (40 MB) or one instead of the two
+    of the GGA's components (100 MB)."""
+    s = systems.si512().band_sample(32)
+    out = []
+    for env in ({}, {"QBX_FAST_ZBUF_MB": str(mb), "QBX_PSIR": psir}):
+        ctx = _ctx(s, monkeypatch, env, precision)
+        out.append((_fields(ctx), [ctx.scf_step()["etotal"] for _ in range(2)]))
+        ctx.close()
+    (fa, sa), (fb, sb) = out
+    tol = 1e-12 if precision == capi.FP64 else 2e-6
+    for a, b in zip(fa[:3], fb[:3]):
+        np.testing.assert_allclose(b, a, rtol=0, atol=tol * np.abs(a).max())
+    np.testing.assert_allclose(sb, sa, rtol=1e-11 if precision == capi.FP64 else 1e-7)
+
+
+@pytest.mark.parametrize("route", ["buffer", "sphere"])
+def test_k_points_on_x_fastest_grids(route, monkeypatch):
+    """k points through the passes that transpose: the stick buffer too small for
+    the density basis, or another k point of the set whose sphere reaches beyond
+    the line kernels' points; against the runtime-radix kernels (FP64)."""
+    far = (2.0, 0.0, 0.0) if route == "sphere" else (0.0, 0.5, 0.4)
+    s = _cell().with_kpoints([((0.25, 0.25, 0.25), 0.5), (far, 0.5)])
+    out = []
+    for env in ({"QBX_FAST_FFT": "0"}, ROUTES[1] if route == "buffer" else {}):
+        ctx = _ctx(s, monkeypatch, env)
+        ctx.update_density()
+        ctx.update_vhxc()
+        e = ctx.energy(hpsi=True)
+        out.append((ctx.density(), ctx.vr(), [ctx.get_kpoint_hpsi(i) for i in range(2)],
+                    e["ekin"], [ctx.scf_step()["etotal"] for _ in range(2)]))
+        ctx.close()
+    (ra, va, ha, ka, ea), (rb, vb, hb, kb, eb) = out
+    for a, b in [(ra, rb), (va, vb)] + list(zip(ha, hb)):
+        np.testing.assert_allclose(b, a, rtol=0, atol=1e-12 * np.abs(a).max())
+    assert abs(ka - kb) <= 1e-11 * abs(ka)
+    np.testing.assert_allclose(eb, ea, rtol=1e-11)

@@ -80,6 +80,28 @@ def test_singular_overlap_is_an_error(precision):
     ctx.close()
 
 
+@pytest.mark.parametrize("n", [16, 45, 128])
+def test_pivots_over_their_range(n):
+    """Bands scaled by powers of two, the pivots of their overlap between 1e-35 and
+    1e35 (past both ends of the range in which the kernel takes its own
+    reciprocal square root): every other operation scales exactly, so the aligned
+    bands are those of the unscaled ones to the roundings of the pivots, a few
+    eps each over n of them."""
+    ctx = _ctx(n, capi.FP64, "1")
+    c = ctx.get_coeffs()
+    rng = np.random.default_rng(n)
+    near = c + 0.01 * rng.standard_normal((n, 1)) * np.roll(c, 1, axis=0)
+    scale = np.concatenate([[58, -58, 50, 49, -49, -50], np.linspace(-58, 58, n)])[:n]
+    scale = 2.0 ** rng.permutation(np.round(scale))
+    out = []
+    for f in (np.ones(n), scale):
+        ctx.set_coeffs(near * f[:, None])
+        ctx.ortho_align(c)
+        out.append(ctx.get_coeffs())
+    ctx.close()
+    np.testing.assert_allclose(out[1], out[0], rtol=0, atol=8 * n * np.finfo(float).eps)
+
+
 @pytest.mark.parametrize("n", [1, 31, 33, 65, 200, 432])
 def test_lower_inverse_with_smaller_last_blocks(n):
     """L^-1 by blocks whose last ones are not whole: n eps times the factor's
