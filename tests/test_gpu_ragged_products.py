@@ -42,3 +42,32 @@ def test_ragged_products(bands):
     np.testing.assert_allclose(fa, fb, rtol=0, atol=2e-6 * max(1.0, np.abs(fb).max()))
     np.testing.assert_allclose(ha, hb, rtol=0, atol=2e-6 * np.abs(hb).max())
     np.testing.assert_allclose(ca, cb, rtol=0, atol=2e-5 * np.abs(cb).max())
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_captured_ragged_steps(batch):
+    """Captured steps of ragged band counts, with and without forces and in any
+    order, take the workspaces that their first, eager run sized: the eager
+    steps' energies and forces (1e-7 of them: atomic sums through three steps)."""
+    systems_ = []
+    for bands, edge in ((33, 11.0), (130, 12.5)):
+        pos = systems.diamond_supercell(10.26, 1, 0.03, 4)[:7]
+        systems_.append(systems.System("box", np.diag([edge, 11.5, 12.0]), [systems.SI],
+                                       [(0, p) for p in pos], 20.0, bands, "PBE", 11))
+    order = [False, False, False, True, True, True, False, True]
+    runs = []
+    for graph in (False, True):
+        ctxs = [capi.from_system(s, precision=capi.MIXED) for s in systems_]
+        rows = []
+        for c in ctxs:
+            c.set_step_graph(graph)
+        for forces in order:
+            if batch and graph:
+                rows.append([e["etotal"] for e in capi.scf_step_batch(ctxs, forces=forces)])
+            else:
+                e = [c.scf_step(forces=forces) for c in ctxs]
+                rows.append([x["etotal"] for x in e])
+        runs.append(np.array(rows))
+        for c in ctxs:
+            c.close()
+    np.testing.assert_allclose(runs[1], runs[0], rtol=1e-7)
