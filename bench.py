@@ -317,7 +317,7 @@ def run_ours(args):
     npairs = (s.nbands + 1) // 2
     # the x pass takes all band pairs in one launch
     t_xy, n_xy = prof["xy_vpsi"]["ms_per_step"], prof["xy_vpsi"]["launches_per_step"]
-    bytes_hpsi = algorithmic_bytes_xy_vpsi(mix, npairs, n_xy, 8, 4)
+    bytes_hpsi = algorithmic_bytes_xy_vpsi(mix, npairs, n_xy, 8, 8)
     per_launch_bytes = bytes_hpsi / max(1e-9, n_xy)
     per_launch_ms = t_xy / max(1e-9, n_xy)
     peaks = {}

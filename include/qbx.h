@@ -452,11 +452,11 @@ int qbx_density_static(qbx_context* ctx, const double* d_c, int nst,
                        const double* occ, double* d_rho);
 
 /* No counterpart in the reference (its FFT plans are fixed at build time).
- * Chooses the staged-FFT launch configuration for this context's grid,
- * basis and precision by timing the candidate plane kernels, CTA shapes,
- * band-pair batches and z-stick blocking on the context's own data (after
- * qbx_set_atoms and qbx_set_coeffs).  A summary of the timings and the
- * choice is written to report (report_len bytes, may be NULL). */
+ * Times H psi and the density of this context's wavefunctions (after
+ * qbx_set_atoms and qbx_set_coeffs) and names the kernels that run them, which
+ * the grid and the basis decide: the line passes or the runtime-radix kernels.
+ * It changes nothing but that captured steps are recorded anew.  Timings and
+ * names are written to report (report_len bytes, may be NULL). */
 int qbx_autotune(qbx_context* ctx, char* report, int report_len);
 
 /* Host-only setup helpers (no GPU needed), exposing the same host code the

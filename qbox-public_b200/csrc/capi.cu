@@ -1293,7 +1293,7 @@ int qbx_autotune(qbx_context* h, char* report, int report_len) {
   return guarded(h, [&](Context& c) {
     check_ready(c, true);
     std::vector<std::pair<std::string, double>> log;
-    drop_graphs(c);   // the launch shapes may change
+    drop_graphs(c);   // the timed passes run eagerly; captured steps are recorded anew
     const std::string pick = autotune_fft(c, &log);
     if (report && report_len > 0) {
       std::string r;

@@ -10,8 +10,9 @@
 //
 //   k_zfft_bwd, k_xy, k_zfft_fwd : one CTA per z plane, mixed-radix (2, 3, 4, 5, 7,
 //                11) self-sorting Stockham passes over shared memory with a twiddle
-//                table exp(+2 pi i k/n) built in FP64: grids with a length above
-//                256, and qbx_density_static
+//                table exp(+2 pi i k/n) built in FP64: grids with a length below 16 or
+//                above 256, spheres wider than prune_width (some k points), a slot
+//                larger than the stick buffer, QBX_FAST_FFT=0, qbx_density_static
 //   k_line_fft : the lines of a whole grid, the same passes
 #include <algorithm>
 #include <complex>

@@ -885,7 +885,7 @@ QBX_PENCIL_DECLARE(7)
 // gains of its three axes carries no systematic charge or energy error.
 double pencil_gain_fp32(int n);
 
-// The lengths an FFT grid can have up to 256: even 2^a 3^{0..2} 5^{0,1}
+// The lengths an FFT grid can have from 16 to 256: even 2^a 3^{0..2} 5^{0,1}
 // 7^{0,1} 11^{0,1}.
 inline bool pencil_length(int n) {
   for (int x : {16, 18, 20, 22, 24, 28, 30, 32, 36, 40, 42, 44, 48, 56, 60, 64, 66, 70, 72, 80,

@@ -136,8 +136,7 @@ __global__ void k_pbe(const double* __restrict__ rho, const double* __restrict__
   }
 }
 
-// out(G) = i gx_j(G) scale in(G)
-// out_j = i G_j in scale for the three components (gx: x, y and z blocks of ng)
+// out_j(G) = i G_j in(G) scale for the three components (gx: x, y and z blocks of ng)
 __global__ void k_mul_igx3(const double2* __restrict__ in, const double* __restrict__ gx, int ng,
                            double scale, double2* __restrict__ out) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ng; i += gridDim.x * blockDim.x) {
@@ -161,14 +160,6 @@ __global__ void k_sum_igx3(const double2* __restrict__ a, const double2* __restr
     out[i] = make_double2(-im, re);
   }
 }
-
-__global__ void k_mul(const double* __restrict__ a, const double* __restrict__ b, size_t n,
-                      double* __restrict__ out) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x)
-    out[i] = a[i] * b[i];
-}
-
 
 // sum_i x_i y_i
 struct DotF {

@@ -518,8 +518,8 @@ void ortho_align(Context& ctx, bool c_split_done) {
     ProfScope ps(ctx, "polar");
     ortho_small(ctx, L, X, X, mx ? ctx.d_nn3 : nullptr, ST_INFO_ORTHO);
   } else if (mx) {
-    // L^-1 once (one triangular solve of I), then two products in place of
-    // the two solves with L and L^T (each solve as slow as the inverse)
+    // L^-1 once, by blocks, then two products in place of the two solves with
+    // L and L^T (each solve slower than the inverse)
     double* Li = ctx.d_nn5;
     double* T = L;   // L is not read after L^-1 is formed
     lower_inverse(ctx, L, n, Li, ctx.d_nn3);   // d_nn3 is free until the rotation

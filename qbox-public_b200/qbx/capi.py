@@ -514,8 +514,8 @@ class Context:
         return n.value, launches.value, batch.value, buf.value.decode()
 
     def autotune(self) -> str:
-        """qbx_autotune: time the staged-FFT configurations on this context
-        and keep the fastest; returns the report."""
+        """qbx_autotune: time H psi and the density on this context and name the
+        kernels that run them; returns the report."""
         buf = ctypes.create_string_buffer(4096)
         self._ok(self.lib.qbx_autotune(self.h, buf, 4096), "autotune")
         return buf.value.decode()
