@@ -329,13 +329,13 @@ def run_ours(args):
     achieved = per_launch_bytes / (per_launch_ms * 1e-3) / 1e9
     roofline = {"kernel": "pen::xv<float, 140> (H*psi x pass: x transform of the tiles kept "
                           "from the density pass, times V, transform back in place)",
-                "bound": "hbm",
+                "bound": "issue",   # 60 % of the slots; DRAM at 31 % (profiles/)
                 "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                 "frac": achieved / hbm_peak,
                 "peak_source": "measured" if "hbm_gbs" in peaks else "fallback",
-                # every tile element is read and written by one thread, so
-                # the DRAM bytes are the algorithmic ones
-                "traffic": per_launch_bytes,
+                # DRAM bytes of the ncu capture (profiles/fft_pencil_si512.md:
+                # 645.7 MB for 32 band pairs) scaled by the band pairs
+                "traffic": 645.7e6 / 32.0 * (npairs / max(1e-9, n_xy)),
                 "algorithmic_bytes_per_launch": per_launch_bytes,
                 "launch_ms": per_launch_ms}
     # GEMM share: the split-precision products of the mixed step (BF16 and
@@ -621,7 +621,7 @@ def run_ours(args):
 def run_profile_case(args):
     """A case for ncu: the 512-atom cell with a band sample (all 1024 bands
     for the launch list of the headline step; 64 for full captures, whose
-    plane kernels do the same work per launch while the device holds a few
+    kernels do the same work per band pair while the device holds a few
     GB), mixed precision.  Warm-up steps run before cudaProfilerStart, so
     `ncu --profile-from-start off` sees exactly one electronic step."""
     import torch

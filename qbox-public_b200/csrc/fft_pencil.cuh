@@ -34,7 +34,7 @@
 // for every other grid and for k points, runtime-radix kernels.  What bounds
 // them now is HBM for the y passes (80 % of the measured copy rate at 140^3)
 // and FP32 issue with the shared-memory exchange for xv.  Per step, density +
-// H psi, before and after (ms): 512 atoms 140^3 FP32 15.5 -> 10.6, FP64 94.7 ->
+// H psi, before and after (ms): 512 atoms 140^3 FP32 15.5 -> 10.8, FP64 94.7 ->
 // 21.1; 64 atoms 84^3 FP32 0.70 -> 0.40, FP64 2.24 -> 0.67; 112 x 72 x 40 FP32
 // 1.09 -> 0.23; two k points 84^3 FP64 13.4 -> 2.4.
 #pragma once
